@@ -235,37 +235,71 @@ __device__ __forceinline__ uint2 bc1_encode_cta(bool valid, const uint32_t t[16]
 }
 
 // ---------------------------------------------------------------- BC4 (zap_tex.h:170-213)
+// round(a b) for |a b| < 2^22: the sum with 1.5 * 2^23 is rounded to an integer, and taking that away is exact
+ZTC_DEV float bc4_rint_mul(float a, float b) { return fma_rn(a, b, 12582912.0f) - 12582912.0f; }
+
+// Plus or minus the distance of a level v to the nearest of the eight palette levels a1 + round(m D / 7), m = 0..7
+// (D = a0 - a1 > 0), from u = 7 (v - a1) and i7 = 1 / (7 D), without the palette. With r = u - m D the distance
+// to level m is round(|r| / 7) (an integer over 7 never ties), so the nearest level is one of least |r|: m = round(u / D),
+// clamped to 0..7 for a v outside [a1, a0]. u / D as computed is within 1e-5 of exact, and exactly it is either a
+// half (both neighbours then have the same |r|) or at least 1 / (2 * 255) away from one, so the rounding is right
+// for every i7 within a few ulp.
+ZTC_DEV float bc4_distance(float u, float D, float i7) {
+    const float m = bc4_rint_mul(saturate(u * i7), 7.0f);
+    return bc4_rint_mul(fma_rn(-m, D, u), 1.0f / 7.0f);
+}
+
+// The reference scans the 8-level palettes of 9 inset endpoint pairs for all 16 texels, keeping the best pair's indices.
+// Here a pair's SSE comes from bc4_distance (8 float operations per texel instead of a scan of about 28 integer
+// ones; integer-valued float sums below 2^24 are exact), one minimum over (SSE, pair) picks the pair, and only that
+// pair's palette is scanned for indices (the lower one on ties, as the reference's scan keeps).
 ZTC_DEV uint2 bc4_encode(const uint32_t t[16], int c) {
-    int v[16], lo = 255, hi = 0;
+    float f[16], lo = 1785.0f, hi = 0.0f;  // 7 v
     #pragma unroll
-    for (int i = 0; i < 16; i++) { v[i] = (int)chan(t[i], c); lo = min(lo, v[i]); hi = max(hi, v[i]); }
-    int best = 1 << 30, ba0 = hi, ba1 = lo;
-    uint64_t bidx = 0;
-    for (int cand = 0; cand < 9; cand++) {
-        int a0 = hi - cand / 3, a1 = lo + cand % 3;
-        if (a0 <= a1) { a0 = hi; a1 = lo; }
-        int err = 0;
-        uint64_t bits = 0;
-        if (a0 == a1) {
-            #pragma unroll
-            for (int i = 0; i < 16; i++) err += (v[i] - a0) * (v[i] - a0);
-        } else {
-            int p[8];
-            p[0] = a0; p[1] = a1;
-            #pragma unroll
-            for (int k = 2; k < 8; k++) p[k] = ((8 - k) * a0 + (k - 1) * a1 + 3) / 7;
-            #pragma unroll
-            for (int i = 0; i < 16; i++) {
-                int m = 1 << 30;
-                #pragma unroll
-                for (int k = 0; k < 8; k++) { int d = v[i] - p[k]; m = min(m, d * d * 8 + k); }
-                err += m >> 3;
-                bits |= (uint64_t)(m & 7) << (3 * i);
-            }
-        }
-        if (err < best) { best = err; ba0 = a0; ba1 = a1; bidx = bits; }
+    for (int i = 0; i < 16; i++) {
+        f[i] = fma_rn(u_as_f(0x4B000000u | chan(t[i], c)), 7.0f, -58720256.0f);  // 7 (2^23 + v) - 7 * 2^23
+        lo = fminf(lo, f[i]); hi = fmaxf(hi, f[i]);
     }
-    return make_uint2((uint32_t)ba0 | ((uint32_t)ba1 << 8) | ((uint32_t)(bidx & 0xFFFFu) << 16), (uint32_t)(bidx >> 16));
+    float key = 3.0e38f;  // 16 SSE + pair < 2^24
+    #pragma unroll 1
+    for (int j = 0; j < 3; j++) {
+        const float base = lo + 7.0f * (float)j;  // 7 a1
+        float D[3], i7[3], e[3];
+        #pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float d7 = hi - base - 7.0f * (float)k;  // 7 D
+            D[k] = bc4_rint_mul(d7, 1.0f / 7.0f);
+            i7[k] = d7 > 0.0f ? rcp_approx(d7) : 0.0f;
+            e[k] = 0.0f;
+        }
+        #pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const float u = f[i] - base;
+            #pragma unroll
+            for (int k = 0; k < 3; k++) { const float d = bc4_distance(u, D[k], i7[k]); e[k] = fma_rn(d, d, e[k]); }
+        }
+        // a pair without a0 > a1 stands for (hi, lo) again, which is pair 0: left out, except pair 0 of a flat block,
+        // whose distances are u = 0
+        #pragma unroll
+        for (int k = 0; k < 3; k++)
+            if (D[k] > 0.0f || (k == 0 && j == 0)) key = fminf(key, fma_rn(e[k], 16.0f, (float)(3 * k + j)));
+    }
+    const int pair = trunc_i(key) & 15, pk = pair / 3, pj = pair - 3 * pk;
+    const float a1 = lo * (1.0f / 7.0f), a0 = hi * (1.0f / 7.0f);  // within an ulp of an integer: rounded below
+    const int ia0 = (int)(f_as_u(a0 + 8388608.0f) & 0xFFu) - pk, ia1 = (int)(f_as_u(a1 + 8388608.0f) & 0xFFu) + pj;
+    float p[8];  // 8 times the palette, a0, a1, then from a0 to a1
+    #pragma unroll
+    for (int k = 0; k < 8; k++) p[k] = small_u2f((uint32_t)(8 * (k == 0 ? ia0 : k == 1 ? ia1 : ((8 - k) * ia0 + (k - 1) * ia1 + 3) / 7)));
+    uint32_t bits[2] = {0u, 0u};  // texels 0..7 and 8..15, 3 bits each
+    #pragma unroll
+    for (int i = 15; i >= 0; i--) {
+        const float v = fma_rn(u_as_f(0x4B000000u | chan(t[i], c)), 8.0f, -67108864.0f);
+        float m = fabsf(v - p[0]);  // 8 distance + index
+        #pragma unroll
+        for (int k = 1; k < 8; k++) m = fminf(m, fabsf(v - p[k]) + (float)k);
+        bits[i >> 3] = bits[i >> 3] * 8u + (f_as_u(m + 8388608.0f) & 7u);
+    }
+    return make_uint2((uint32_t)ia0 | ((uint32_t)ia1 << 8) | (bits[0] << 16), (bits[0] >> 16) | (bits[1] << 8));
 }
 
 // ---------------------------------------------------------------- kernel: one thread per block

@@ -87,6 +87,8 @@ ZTC_DEV float u_as_f(uint32_t u) { return __uint_as_float(u); }
 ZTC_DEV uint32_t brev(uint32_t v) { return __brev(v); }
 ZTC_DEV int trunc_i(float f) { return __float2int_rz(f); }
 ZTC_DEV float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+ZTC_DEV float saturate(float x) { return __saturatef(x); }
+ZTC_DEV float rcp_approx(float x) { return __fdividef(1.0f, x); }  // within 2 ulp of 1 / x, for |x| below 2^126
 template <typename T> ZTC_DEV T ldg(const T *p) { return __ldg(p); }
 #else
 inline uint32_t dot4(uint32_t a, uint32_t b) {
@@ -100,6 +102,8 @@ inline float u_as_f(uint32_t u) { float f; std::memcpy(&f, &u, 4); return f; }
 inline uint32_t brev(uint32_t v) { uint32_t r = 0; for (int k = 0; k < 32; k++) r |= ((v >> k) & 1u) << (31 - k); return r; }
 inline int trunc_i(float f) { return (int)f; }  // only called on in-range values
 inline float fma_rn(float a, float b, float c) { return std::fmaf(a, b, c); }
+inline float saturate(float x) { return x > 1.0f ? 1.0f : x > 0.0f ? x : 0.0f; }
+inline float rcp_approx(float x) { return 1.0f / x; }
 template <typename T> inline T ldg(const T *p) { return *p; }
 #endif
 
@@ -280,6 +284,33 @@ ZTC_DEV void gather_block(const SrcU8 &s, int bx, int by, uint32_t t[16]) {
             t[4 * r + 0] = v.x; t[4 * r + 1] = v.y; t[4 * r + 2] = v.z; t[4 * r + 3] = v.w;
         }
         return;
+    }
+    if (x0 + 3 < s.w && y0 + 3 < s.h) {  // a whole block at a lesser alignment: rows of plain words
+        const uint8_t *p = s.base + (size_t)y0 * s.stride + (size_t)x0 * (size_t)s.channels;
+        const uint32_t align = (uint32_t)((uintptr_t)s.base | s.stride);
+        if (s.channels == 4 && (align & 3u) == 0) {
+            #pragma unroll
+            for (int i = 0; i < 16; i++) t[i] = ldg((const uint32_t *)(p + (size_t)(i >> 2) * s.stride) + (i & 3));
+            return;
+        }
+        if (s.channels == 2 && (align & 7u) == 0) {
+            #pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const uint2 v = ldg((const uint2 *)(p + (size_t)r * s.stride));
+                t[4 * r + 0] = (v.x & 0xFFFFu) | 0xFF000000u; t[4 * r + 1] = (v.x >> 16) | 0xFF000000u;
+                t[4 * r + 2] = (v.y & 0xFFFFu) | 0xFF000000u; t[4 * r + 3] = (v.y >> 16) | 0xFF000000u;
+            }
+            return;
+        }
+        if (s.channels == 1 && (align & 3u) == 0) {
+            #pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const uint32_t v = ldg((const uint32_t *)(p + (size_t)r * s.stride));
+                #pragma unroll
+                for (int k = 0; k < 4; k++) t[4 * r + k] = ((v >> (8 * k)) & 0xFFu) | 0xFF000000u;
+            }
+            return;
+        }
     }
     #pragma unroll
     for (int i = 0; i < 16; i++) {
