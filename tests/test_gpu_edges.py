@@ -1,0 +1,54 @@
+"""Edges of the kernels' tiles and of the sizes their launch rules turn on, against the oracle, byte for byte."""
+import numpy as np
+import pytest
+import torch
+
+import zap_b200
+
+pytestmark = pytest.mark.gpu
+
+
+def _image(w, h, seed):
+    """Half smooth, half noise, in a row pitch of its own (as a view when `w` is odd)."""
+    rng = np.random.default_rng(seed)
+    img = rng.integers(0, 256, (h, w, 4), dtype=np.uint8)
+    img[: (h + 1) // 2] = np.sort(img[: (h + 1) // 2], axis=1)
+    return img
+
+
+@pytest.mark.parametrize("size", [(1, 1), (1, 9), (70, 1), (64, 64), (65, 63), (127, 130), (3, 300), (129, 256), (640, 71), (1030, 517)])
+@pytest.mark.parametrize("srgb", [0, 1])
+def test_mip_chain_edges(cuda_lib, oracle, size, srgb):
+    """Chains around the 64x64 tile and the six levels of a launch; 16-byte, 4-byte and 1-byte aligned rows."""
+    w, h = size
+    for pad in (0, 1):  # pad: the image as a view of wider rows, one texel in
+        img = _image(w, h, 10 * w + h + srgb)
+        wide = torch.zeros(h, w + 2 * pad, 4, dtype=torch.uint8, device="cuda")
+        wide[:, pad:pad + w] = torch.from_numpy(img).cuda()
+        view = wide[:, pad:pad + w]
+        want, got = img, zap_b200.mip_chain_dev(view, srgb)
+        for level in got:
+            want = oracle.mip_next(want, srgb)
+            assert np.array_equal(level.cpu().numpy(), want), (size, srgb, pad, want.shape)
+        if max(w, h) > 1:
+            assert np.array_equal(zap_b200.mip_next_dev(view, srgb).cpu().numpy(), oracle.mip_next(img, srgb))
+
+
+@pytest.mark.parametrize("fmt,channels", [(zap_b200.BC4, 1), (zap_b200.BC5, 2), (zap_b200.BC4, 4), (zap_b200.BC3, 4)])
+@pytest.mark.parametrize("size", [(4, 4), (7, 5), (36, 12), (1000, 600)])
+def test_channel_blocks(cuda_lib, oracle, fmt, channels, size):
+    """Flat blocks, ranges from 1 to 255 levels (palettes with repeated entries below 7), every row alignment."""
+    w, h = size
+    rng = np.random.default_rng(w + fmt)
+    bw, bh = (w + 3) // 4, (h + 3) // 4
+    lo = np.kron(rng.integers(0, 256, (bh, bw)), np.ones((4, 4), int))[:h, :w]
+    span = np.kron((256.0 ** rng.random((bh, bw))).astype(int) - 1, np.ones((4, 4), int))[:h, :w]
+    img = np.zeros((h, w, 4), np.uint8)
+    img[..., 3] = 255
+    for c in ((0, 1, 3) if channels == 4 else range(channels)):
+        img[..., c] = np.clip(lo + (rng.random((h, w)) * (span + 1)).astype(int), 0, 255)
+    for x0 in (0, 1):  # a view one texel in: the next alignment down
+        sub = np.ascontiguousarray(img[:, x0:])
+        t = torch.from_numpy(img[..., :channels].copy()).cuda()[:, x0:]
+        if sub.shape[1]:
+            assert np.array_equal(zap_b200.bc_encode_dev(t, fmt).cpu().numpy(), oracle.bc_encode(sub, fmt)), (fmt, size, x0)

@@ -771,12 +771,17 @@ int zap_tex_cuda_mip_chain_dev(zap_tex_cuda_ctx *ctx, const uint8_t *rgba, int w
     const uint8_t *prev = rgba;
     size_t prev_stride = stride;
     uint8_t *o = dst;
-    while (w > 1 || h > 1) {
-        int nw = w > 1 ? w / 2 : 1, nh = h > 1 ? h / 2 : 1;
-        cudaError_t e = ztc_launch_mip(prev, w, h, prev_stride, srgb, o, (size_t)nw * 4, (cudaStream_t)stream);
+    while (w > 1 || h > 1) {  // six levels a launch
+        ztc::MipChain c{};
+        c.src = prev; c.pitch = prev_stride; c.w = w; c.h = h; c.srgb = srgb ? 1 : 0;
+        for (; c.levels < ztc::kMipLevels && (w > 1 || h > 1); c.levels++) {
+            w = w > 1 ? w / 2 : 1; h = h > 1 ? h / 2 : 1;
+            if (!c.levels) c.dst_pitch = (size_t)w * 4;
+            c.dst[c.levels] = o;
+            prev = o; prev_stride = (size_t)w * 4; o += (size_t)w * h * 4;
+        }
+        const cudaError_t e = ztc_launch_mip_levels(c, (cudaStream_t)stream);
         if (e != cudaSuccess) return cuda_fail(e, "mip launch");
-        prev = o; prev_stride = (size_t)nw * 4; o += (size_t)nw * nh * 4;
-        w = nw; h = nh;
     }
     return ZTC_OK;
 }

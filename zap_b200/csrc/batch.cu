@@ -2,8 +2,8 @@
 //
 // No single reference counterpart: it replaces the caller loop of zap.c:330-342 (per level: zap_bc_encode, then
 // zap_mip_next) run over many textures. A batch is planned once (zap_tex_cuda_batch_create):
-//   - mip levels 1..L-1 of every texture go to one device buffer; depth d of all textures is built by one
-//     persistent launch over tiles of 256 output texel pairs (level-synchronous, L-1 launches in all);
+//   - mip levels 1..L-1 of every texture go to one device buffer; six depths of all textures are built by one
+//     persistent launch over 64x64 source tiles (mip.cu; two launches for chains from 4096x4096);
 //   - every (texture, level) is cut into tiles of consecutive blocks; one persistent launch per format class pulls
 //     tiles from a device counter (largest levels first); for BC7 that launch runs mode 6 and lists the blocks it
 //     does not finish in one batch-wide work list, which a second persistent launch (8-lane groups, modes 5 / 1)
@@ -59,22 +59,21 @@ struct zap_tex_cuda_batch {
     cudaStream_t stream = nullptr, side[kClasses] = {};
     cudaEvent_t fork = nullptr, join[kClasses] = {};
     std::vector<HostLevel> levels;          // every (item, level), item-major
-    std::vector<std::vector<ztc::BatchMip>> mips;  // per depth d >= 1
+    std::vector<std::vector<ztc::MipChain>> mips;  // per launch of six depths
     uint8_t *mip_buf = nullptr;
     size_t mip_bytes = 0;
     ztc::BatchLevel *d_levels = nullptr;
     ztc::BatchTile *d_tiles[kClasses] = {};
     int ntiles[kClasses] = {}, grid[kClasses] = {};
     ClassPlan plan[kClasses];
-    std::vector<ztc::BatchMip *> d_mips;
-    std::vector<ztc::BatchMipTile *> d_mip_tiles;
+    std::vector<ztc::MipChain *> d_mips;
+    std::vector<ztc::MipTile *> d_mip_tiles;
     std::vector<int> n_mip_tiles;
     uint32_t *d_counters = nullptr;          // [f]: tile counter of class f; [kHardCounter]: BC7 work-list length
     uint2 *d_hard_items = nullptr;           // BC7 work lists: (batch-wide block id, SSE) after mode 6, then after mode 5
     uint32_t *d_bc7_bases = nullptr;         // first batch-wide id of each BC7 level, ascending
     int *d_bc7_level_of = nullptr;           // ... and that level's index in d_levels
     int n_bc7_levels = 0, hard_grid = 1, hard_per_sm = 1;
-    ztc::SrgbTables *d_srgb = nullptr;
     void *plain_scratch = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -169,10 +168,10 @@ cudaError_t launch_mips(zap_tex_cuda_batch *b, cudaStream_t s) {
         if (!b->n_mip_tiles[d]) continue;
         ztc::TraceScope tr("batch_mip", s);
         long units = 0;
-        for (auto &m : b->mips[d]) units += (long)m.nw * m.nh;
+        for (auto &m : b->mips[d])
+            for (int l = 1; l <= m.levels; l++) units += (long)std::max(1, m.w >> l) * std::max(1, m.h >> l);
         ztc::trace_units(units);
-        int grid = std::max(1, std::min(b->n_mip_tiles[d], b->sms * 8));
-        cudaError_t e = ztc_launch_batch_mip(grid, b->d_mips[d], b->d_mip_tiles[d], b->n_mip_tiles[d], b->d_srgb, s);
+        cudaError_t e = ztc_launch_batch_mip(b->d_mips[d], b->d_mip_tiles[d], b->n_mip_tiles[d], s);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -296,7 +295,7 @@ int zap_tex_cuda_batch_destroy(zap_tex_cuda_batch *b) {
     }
     for (auto p : b->d_mips) cudaFree(p);
     for (auto p : b->d_mip_tiles) cudaFree(p);
-    cudaFree(b->mip_buf); cudaFree(b->d_levels); cudaFree(b->d_counters); cudaFree(b->d_srgb); cudaFree(b->plain_scratch);
+    cudaFree(b->mip_buf); cudaFree(b->d_levels); cudaFree(b->d_counters); cudaFree(b->plain_scratch);
     cudaFree(b->d_hard_items); cudaFree(b->d_bc7_bases); cudaFree(b->d_bc7_level_of);
     if (b->fork) cudaEventDestroy(b->fork);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -367,29 +366,37 @@ int zap_tex_cuda_batch_create(zap_tex_cuda_ctx *ctx, const zap_tex_cuda_item *it
         if (hl.level == 0) { hl.src = items[hl.item].src; hl.pitch = items[hl.item].stride; }
         else { hl.src = b->mip_buf + mip_off[k]; hl.pitch = (size_t)hl.w * 4; }
     }
-    // ---- mip work per depth
-    b->mips.resize(max_levels > 1 ? max_levels - 1 : 0);
+    // ---- mip work per launch: levels 6g + 1 .. 6g + 6 of each item from its level 6g
+    b->mips.resize((max_levels - 1 + ztc::kMipLevels - 1) / ztc::kMipLevels);
     for (size_t k = 0; k < b->levels.size(); k++) {
         const HostLevel &hl = b->levels[k];
         if (hl.level == 0) continue;
-        const HostLevel &prev = b->levels[k - 1];
-        b->mips[hl.level - 1].push_back({prev.src, (uint8_t *)hl.src, prev.pitch, hl.pitch, prev.w, prev.h, hl.w, hl.h, hl.srgb, 0});
-    }
-    for (auto &depth : b->mips) {
-        std::vector<ztc::BatchMipTile> tiles;
-        for (int m = 0; m < (int)depth.size(); m++) {
-            int pairs = ((depth[m].nw + 1) / 2) * depth[m].nh;
-            for (int first = 0; first < pairs; first += 256) tiles.push_back({m, first, std::min(256, pairs - first), 0});
+        std::vector<ztc::MipChain> &group = b->mips[(hl.level - 1) / ztc::kMipLevels];
+        if ((hl.level - 1) % ztc::kMipLevels == 0) {
+            const HostLevel &prev = b->levels[k - 1];
+            ztc::MipChain c{};
+            c.src = prev.src; c.pitch = prev.pitch; c.dst_pitch = hl.pitch; c.w = prev.w; c.h = prev.h; c.srgb = hl.srgb;
+            group.push_back(c);
         }
-        ztc::BatchMip *dm = nullptr;
-        ztc::BatchMipTile *dt = nullptr;
-        BTRY(ztc_malloc((void **)&dm, std::max<size_t>(1, depth.size()) * sizeof(ztc::BatchMip)), "cudaMalloc(mips)");
+        ztc::MipChain &c = group.back();
+        c.dst[c.levels++] = (uint8_t *)hl.src;
+    }
+    for (auto &group : b->mips) {
+        std::vector<ztc::MipTile> tiles;
+        for (int m = 0; m < (int)group.size(); m++) {
+            int tx = 1;
+            const int n = ztc::mip_tiles(group[m].w, group[m].h, tx);
+            for (int t = 0; t < n; t++) tiles.push_back({m, t % tx, t / tx, 0});
+        }
+        ztc::MipChain *dm = nullptr;
+        ztc::MipTile *dt = nullptr;
+        BTRY(ztc_malloc((void **)&dm, std::max<size_t>(1, group.size()) * sizeof(ztc::MipChain)), "cudaMalloc(mips)");
         b->d_mips.push_back(dm);
-        BTRY(ztc_malloc((void **)&dt, std::max<size_t>(1, tiles.size()) * sizeof(ztc::BatchMipTile)), "cudaMalloc(mip tiles)");
+        BTRY(ztc_malloc((void **)&dt, std::max<size_t>(1, tiles.size()) * sizeof(ztc::MipTile)), "cudaMalloc(mip tiles)");
         b->d_mip_tiles.push_back(dt);
         b->n_mip_tiles.push_back((int)tiles.size());
-        if (!depth.empty()) BTRY(cudaMemcpy(dm, depth.data(), depth.size() * sizeof(ztc::BatchMip), cudaMemcpyHostToDevice), "upload mips");
-        if (!tiles.empty()) BTRY(cudaMemcpy(dt, tiles.data(), tiles.size() * sizeof(ztc::BatchMipTile), cudaMemcpyHostToDevice), "upload mip tiles");
+        if (!group.empty()) BTRY(cudaMemcpy(dm, group.data(), group.size() * sizeof(ztc::MipChain), cudaMemcpyHostToDevice), "upload mips");
+        if (!tiles.empty()) BTRY(cudaMemcpy(dt, tiles.data(), tiles.size() * sizeof(ztc::MipTile), cudaMemcpyHostToDevice), "upload mip tiles");
     }
     // ---- level descriptors, tables, counters
     std::vector<ztc::BatchLevel> dl;
@@ -426,10 +433,6 @@ int zap_tex_cuda_batch_create(zap_tex_cuda_ctx *ctx, const zap_tex_cuda_item *it
         b->hard_per_sm = std::max(1, per_sm);
         b->hard_grid = b->hard_per_sm * b->sms;
     }
-    ztc::SrgbTables tables;
-    ztc::srgb_tables_host(tables);
-    BTRY(ztc_malloc((void **)&b->d_srgb, sizeof tables), "cudaMalloc(srgb)");
-    BTRY(cudaMemcpy(b->d_srgb, &tables, sizeof tables, cudaMemcpyHostToDevice), "upload srgb");
     BTRY(ztc_malloc((void **)&b->d_counters, 64 * sizeof(uint32_t)), "cudaMalloc(counters)");
     BTRY(ztc_malloc((void **)&b->plain_scratch, ztc::bc7_scratch_bytes(max_blocks)), "cudaMalloc(plain scratch)");
     // ---- tiles (autotuned or 128 blocks per CTA)

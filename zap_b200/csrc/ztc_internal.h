@@ -71,15 +71,17 @@ __host__ __device__ inline int tile_block(const BatchTile &t, int bw, int j) {
     return t.tw ? t.first + (j / t.tw) * bw + (j % t.tw) : t.first + j;
 }
 #endif
-struct BatchMip {       // one (texture, level d >= 1): built from level d - 1
-    const uint8_t *src;
-    uint8_t *dst;
-    size_t src_pitch, dst_pitch;
-    int w, h, nw, nh, srgb, pad;  // w, h: source level size
+// Up to six levels of one texture's mip chain, built by one launch from the level above them (mip.cu)
+constexpr int kMipLevels = 6;
+struct MipChain {
+    const uint8_t *src;        // the source level, RGBA8, `pitch` bytes per row
+    size_t pitch, dst_pitch;   // dst_pitch: bytes per row of the first level made; the others are packed (4 * width)
+    uint8_t *dst[kMipLevels];
+    int w, h, levels, srgb;    // w, h: the source level's size
 };
-struct BatchMipTile {   // output texel pairs [first, first + count) of one BatchMip, row-major over (nw + 1) / 2 pairs
-    int mip, first, count, pad;
-};
+struct MipTile { int chain, x, y, pad; };  // one 64x64 source tile of one chain
+// 64x64 source tiles of a level (tiles_x: per row of tiles)
+int mip_tiles(int w, int h, int &tiles_x);
 }  // namespace ztc
 
 // `regs`: 0 = the register cap of the single-image kernels (more resident CTAs), 1 = a looser cap (fewer spills)
@@ -94,21 +96,21 @@ cudaError_t ztc_launch_batch_bc7_mode6(int cta, int regs, int grid, const ztc::B
 cudaError_t ztc_launch_batch_bc7_hard(int grid, const ztc::BatchLevel *levels, const uint32_t *bases, const int *level_of, int nlevels,
                                       const uint32_t *hard_count, const uint2 *hard_items, uint32_t *opaque_count, uint2 *opaque_items,
                                       cudaStream_t stream);
-namespace ztc { struct SrgbTables; }
-cudaError_t ztc_launch_batch_mip(int grid, const ztc::BatchMip *mips, const ztc::BatchMipTile *tiles, int ntiles, const ztc::SrgbTables *srgb_tables,
-                                 cudaStream_t stream);
+cudaError_t ztc_launch_batch_mip(const ztc::MipChain *chains, const ztc::MipTile *tiles, int ntiles, cudaStream_t stream);
 const void *ztc_batch_bcn_kernel_fn(int fmt, int cta, int regs);
 const void *ztc_batch_bc7_kernel_fn(int cta, int regs);  // the mode 6 tile-queue kernel
 const void *ztc_batch_bc7_hard_kernel_fn();
-const void *ztc_batch_mip_kernel_fn();
 namespace ztc {
 // The sRGB tables of the mip generator: linear value of each sRGB code (zap_tex.h:1360-1393), the thresholds where
 // a code rounds up (:1394-1427, + an infinite sentinel), and a search start per bucket of linear values (bucket =
 // the float's exponent and top 6 mantissa bits over [2^-16, 1], bucket 0 below): the answer at the bucket's lowest
-// value, a lower bound for every value in it.
+// value, a lower bound for every value in it. back: the one-word search of srgb_back (mip.cu), a word per exponent and
+// top 7 mantissa bits of a sum over [2^-11, 4].
 constexpr int kSrgbBuckets = 17 * 64;
+constexpr int kSrgbBackLow = 0x3A00, kSrgbBack = 13 * 128 + 1;  // high halves of 2^-11 .. 4.0f
 struct SrgbTables {
     float lin[256], thr[256];
+    uint32_t back[kSrgbBack];
     uint8_t bucket[kSrgbBuckets];
 };
 void srgb_tables_host(SrgbTables &t);
@@ -144,6 +146,7 @@ cudaError_t ztc_launch_bc6h(const ztc::SrcHdr &src, int by0, int nby, uint8_t *o
 cudaError_t ztc_launch_astc(const ztc::SrcU8 &src, int by0, int nby, uint8_t *out, void *scratch, cudaStream_t stream);
 // zap_astc_decode (zap_tex.h:1344-1356), device to device; bc 16-byte aligned
 cudaError_t ztc_launch_astc_decode(const uint8_t *bc, int w, int h, uint8_t *out, size_t stride, cudaStream_t stream);
+cudaError_t ztc_launch_mip_levels(const ztc::MipChain &chain, cudaStream_t stream);  // chain.levels levels, one launch
 cudaError_t ztc_launch_mip(const uint8_t *src, int w, int h, size_t stride, int srgb, uint8_t *dst, size_t dst_stride,
                            cudaStream_t stream);
 cudaError_t ztc_launch_mip_f(const float *src, int w, int h, size_t stride, float *dst, size_t dst_stride, cudaStream_t stream);
