@@ -10,13 +10,13 @@
 
 namespace ztc {
 
-__global__ void __launch_bounds__(128) bcn_decode_kernel(int fmt, const uint8_t *__restrict__ bc, int w, int h, uint8_t *__restrict__ out,
-                                                         size_t stride) {
+template <int FMT>
+__global__ void __launch_bounds__(128) bcn_decode_kernel(const uint8_t *__restrict__ bc, int w, int h, uint8_t *__restrict__ out, size_t stride) {
     const int bw = (w + 3) / 4, nblocks = bw * ((h + 3) / 4);
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nblocks) return;
     uint32_t px[16];
-    dec::bcn_block(fmt, bc + (size_t)b * ((fmt == 0 || fmt == 2) ? 8 : 16), px);
+    dec::bcn_block<FMT>(bc + (size_t)b * ((FMT == 0 || FMT == 2) ? 8 : 16), px);
     const bool vec = (((uintptr_t)out | stride) & 15u) == 0, aligned4 = (((uintptr_t)out | stride) & 3u) == 0;
     dec::store_block_rgba8(out, stride, w, h, b % bw, b / bw, px, vec, aligned4);
 }
@@ -25,9 +25,9 @@ __global__ void __launch_bounds__(128) bc6h_decode_kernel(const uint8_t *__restr
     const int bw = (w + 3) / 4, nblocks = bw * ((h + 3) / 4);
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nblocks) return;
-    uint4 v = *(const uint4 *)(bc + (size_t)b * 16);
+    const uint4 v = ldg((const uint4 *)(bc + (size_t)b * 16));
     const uint32_t wd[4] = {v.x, v.y, v.z, v.w};
-    uint16_t px[16][4];
+    uint32_t px[32];
     dec::bc6h_block(wd, px);
     const int bx = b % bw, by = b / bw;
     // a row of four texels inside the image as two 16-byte stores when the image and its pitch (stride halves) are
@@ -39,16 +39,15 @@ __global__ void __launch_bounds__(128) bc6h_decode_kernel(const uint8_t *__restr
         if (y >= h) break;
         uint16_t *row = out + (size_t)y * stride + (size_t)x0 * 4;
         if (vec && x0 + 3 < w) {
-            uint32_t q[8];
-            #pragma unroll
-            for (int k = 0; k < 8; k++) q[k] = (uint32_t)px[4 * r + (k >> 1)][2 * (k & 1)] | ((uint32_t)px[4 * r + (k >> 1)][2 * (k & 1) + 1] << 16);
-            ((uint4 *)row)[0] = make_uint4(q[0], q[1], q[2], q[3]);
-            ((uint4 *)row)[1] = make_uint4(q[4], q[5], q[6], q[7]);
+            ((uint4 *)row)[0] = make_uint4(px[8 * r], px[8 * r + 1], px[8 * r + 2], px[8 * r + 3]);
+            ((uint4 *)row)[1] = make_uint4(px[8 * r + 4], px[8 * r + 5], px[8 * r + 6], px[8 * r + 7]);
             continue;
         }
+        #pragma unroll
         for (int c = 0; c < 4; c++) {
             if (x0 + c >= w) break;
-            for (int k = 0; k < 4; k++) row[4 * c + k] = px[4 * r + c][k];
+            #pragma unroll
+            for (int k = 0; k < 4; k++) row[4 * c + k] = (uint16_t)(px[8 * r + 2 * c + (k >> 1)] >> (16 * (k & 1)));
         }
     }
 }
@@ -75,7 +74,11 @@ cudaError_t launch_decode(Kind k, const void *bc, int w, int h, int fmt, void *r
     const unsigned grid = (unsigned)((nblocks + 127) / 128);
     if (k == kAstc) return ztc_launch_astc_decode((const uint8_t *)bc, w, h, (uint8_t *)rgba, stride, s);
     if (k == kBc6h) ztc::bc6h_decode_kernel<<<grid, 128, 0, s>>>((const uint8_t *)bc, w, h, (uint16_t *)rgba, stride);
-    else ztc::bcn_decode_kernel<<<grid, 128, 0, s>>>(fmt, (const uint8_t *)bc, w, h, (uint8_t *)rgba, stride);
+    else {
+        auto *fn = fmt == ZTC_BC1 ? ztc::bcn_decode_kernel<0> : fmt == ZTC_BC3 ? ztc::bcn_decode_kernel<1> : fmt == ZTC_BC4 ? ztc::bcn_decode_kernel<2>
+                 : fmt == ZTC_BC5 ? ztc::bcn_decode_kernel<3> : ztc::bcn_decode_kernel<4>;
+        fn<<<grid, 128, 0, s>>>((const uint8_t *)bc, w, h, (uint8_t *)rgba, stride);
+    }
     return cudaGetLastError();
 }
 

@@ -172,6 +172,7 @@ ZTC_DEV int lerp64(int a, int b, int w) { return ((64 - w) * a + w * b + 32) >> 
 // and non-negative, so they separate), and bits 6..13 of each field are the channel's value
 struct Lerp4 {
     uint32_t rb, ga, srb, sga;
+    Lerp4() = default;
     ZTC_DEV Lerp4(const int x0[4], const int x1[4]) {  // 8-bit endpoint channels
         rb = (uint32_t)(64 * x0[0] + 32) | ((uint32_t)(64 * x0[2] + 32) << 16);
         ga = (uint32_t)(64 * x0[1] + 32) | ((uint32_t)(64 * x0[3] + 32) << 16);
@@ -181,6 +182,10 @@ struct Lerp4 {
     ZTC_DEV uint32_t at(int w) const {  // the four channels' lerp64 at weight w, as a texel
         const uint32_t a = rb + srb * (uint32_t)w, b = ga + sga * (uint32_t)w;
         return ((a >> 6) & 0x00FF00FFu) | ((b << 2) & 0xFF00FF00u);
+    }
+    ZTC_DEV uint32_t at2(int w, int wa) const {  // R, G, B at weight w, A at weight wa
+        const uint32_t a = rb + srb * (uint32_t)w, b = ga + sga * (uint32_t)w, c = ga + sga * (uint32_t)wa;
+        return ((a >> 6) & 0x00FF00FFu) | ((b << 2) & 0x0000FF00u) | ((c << 2) & 0xFF000000u);
     }
 };
 ZTC_DEV int expand_bits(int v, int n) { v <<= 8 - n; return v | (v >> n); }  // n-bit -> 8-bit replication

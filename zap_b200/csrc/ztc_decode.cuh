@@ -143,70 +143,159 @@ ZTC_DEV bool bc7_parse(const uint32_t w[4], Bc7Fields &F) {
     return true;
 }
 
+// ---------------------------------------------------------------- decode to texels
+// The BC7 interpolation weights (wbits) as j shifted and multiplied: two or three operations.
+template <int IB>
+ZTC_DEV int weight_of(uint32_t j) {
+    return (int)(IB == 2 ? 21u * j + (j >> 1) : IB == 3 ? 9u * j + (j >> 2) : 4u * j + ((j + 2u) >> 2));
+}
+// bits [pos, pos + n) of a block held as two 64-bit words (n <= 63; pos and n are compile-time where it is inlined)
+ZTC_DEV uint64_t field64(uint64_t lo, uint64_t hi, int pos, int n) {
+    const uint64_t v = pos >= 64 ? hi >> (pos - 64) : pos == 0 ? lo : (lo >> pos) | (hi << (64 - pos));
+    return v & ((1ull << n) - 1ull);
+}
+// an index stream with the anchors' missing top bits put back as zeros (p: position of one, the lower ones already
+// back): the bits from p up move up by one
+ZTC_DEV uint64_t open_bit(uint64_t x, int p) { return x + (x & (~0ull << p)); }
+
+// One BC7 block of a mode whose layout is known at compile time (zap_tex.h:378-417): every field at a fixed position,
+// the indices as one 64-bit stream of equal widths, two channels per word in the interpolation. The fields never
+// leave registers: a parse into arrays indexed by run-time field widths kept them in local memory and made a
+// warp with any block outside mode 6 wait for it
+// (2048x2048, 4 % such blocks: 34.3 -> 8.7 us, BC3 10.8 -> 6.7; 3.2 us is the copy bound).
+template <int MODE, int NS, int PB, int RB, int ISB, int CB, int AB, int EPB, int SPB, int IB, int IB2>
+ZTC_DEV void bc7_mode_block(uint64_t lo, uint64_t hi, uint32_t out[16]) {
+    constexpr int kEnds = 2 * NS, kBase = MODE + 1 + PB + RB + ISB, kAlpha = kBase + 3 * kEnds * CB, kP = kAlpha + kEnds * AB;
+    constexpr int kIdx = kP + (EPB ? kEnds : 0) + (SPB ? NS : 0), kIdx2 = kIdx + 16 * IB - NS, kPb = (EPB || SPB) ? 1 : 0;
+    const int part = PB ? (int)field64(lo, hi, MODE + 1, PB) : 0;
+    const uint32_t rot = RB ? (uint32_t)field64(lo, hi, MODE + 1 + PB, RB) : 0u;
+    const bool swap = ISB && field64(lo, hi, MODE + 1 + PB + RB, 1) != 0;
+    Lerp4 row[NS];
+    #pragma unroll
+    for (int s = 0; s < NS; s++) {
+        int x[2][4];
+        #pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int e = 2 * s + k;
+            const int p = EPB ? (int)field64(lo, hi, kP + e, 1) : SPB ? (int)field64(lo, hi, kP + s, 1) : 0;
+            #pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (c == 3 && !AB) { x[k][c] = 255; continue; }
+                const int n = c < 3 ? CB : AB, pos = c < 3 ? kBase + (c * kEnds + e) * CB : kAlpha + e * AB;
+                x[k][c] = expand_bits((int)(field64(lo, hi, pos, n) << kPb) | p, n + kPb);
+            }
+        }
+        row[s] = Lerp4(x[0], x[1]);
+    }
+    uint32_t mask = 0;  // the texels' subsets, one or two bits a texel
+    uint64_t i1 = field64(lo, hi, kIdx, 16 * IB - NS), i2 = 0;
+    i1 = open_bit(i1, IB - 1);
+#ifdef __CUDA_ARCH__
+    if (NS == 2) {
+        mask = kP2d[part];
+        i1 = open_bit(i1, kA2d[part] * IB + IB - 1);
+    } else if (NS == 3) {
+        mask = kP3d[part];
+        const int a = kA3ad[part], b = kA3bd[part];
+        i1 = open_bit(i1, min(a, b) * IB + IB - 1);
+        i1 = open_bit(i1, max(a, b) * IB + IB - 1);
+    }
+#endif
+    if (IB2) i2 = open_bit(field64(lo, hi, kIdx2, 16 * IB2 - 1), IB2 - 1);
+    // rotation: alpha and channel rot - 1 change places after the interpolation
+    const uint32_t sel = rot == 0 ? 0x3210u : rot == 1 ? 0x0213u : rot == 2 ? 0x1230u : 0x2310u;
+    #pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const int w1 = weight_of<IB>((uint32_t)(i1 >> (IB * i)) & ((1u << IB) - 1u));
+        if (IB2) {
+            const int w2 = weight_of<IB2 ? IB2 : 2>((uint32_t)(i2 >> (IB2 * i)) & ((1u << IB2) - 1u));
+            const uint32_t t = row[0].at2(swap ? w2 : w1, swap ? w1 : w2);
+#ifdef __CUDA_ARCH__
+            out[i] = __byte_perm(t, 0u, sel);
+#else
+            out[i] = chan(t, sel & 3) | (chan(t, (sel >> 4) & 3) << 8) | (chan(t, (sel >> 8) & 3) << 16) | (chan(t, (sel >> 12) & 3) << 24);
+#endif
+        } else if (NS == 1) {
+            out[i] = row[0].at(w1);
+        } else {
+            const uint32_t s = NS == 2 ? (mask >> i) & 1u : (mask >> (2 * i)) & 3u;
+            Lerp4 r = s == 0 ? row[0] : row[1];
+            if (NS == 3 && s == 2) r = row[NS - 1];
+            out[i] = r.at(w1);
+        }
+    }
+}
+
 // full BC7 decode, all 8 modes; reserved mode -> transparent black (zap_tex.h:378-417)
 ZTC_DEV void bc7_block(const uint32_t w[4], uint32_t out[16]) {
-    if ((w[0] & 0x7Fu) == 0x40u) {  // mode 6, the encoder's common case, straight from its fixed layout
-        // R0 R1 G0 G1 B0 B1 A0 A1 (7 bits each) from bit 7, p-bits at 63 and 64, indices from bit 65 (texel 0: 3 bits)
-        const uint64_t lo = w[0] | ((uint64_t)w[1] << 32), hi = w[2] | ((uint64_t)w[3] << 32);
-        const int p0 = (int)(lo >> 63), p1 = (int)(hi & 1u);
-        int x0[4], x1[4];
+    const uint64_t lo = w[0] | ((uint64_t)w[1] << 32), hi = w[2] | ((uint64_t)w[3] << 32);
+    const uint32_t m = w[0] & 0xFFu;  // the mode is the place of the lowest set bit
+    if ((m & 0x7Fu) == 0x40u) bc7_mode_block<6, 1, 0, 0, 0, 7, 7, 1, 0, 4, 0>(lo, hi, out);
+    else if ((m & 0x3Fu) == 0x20u) bc7_mode_block<5, 1, 0, 2, 0, 7, 8, 0, 0, 2, 2>(lo, hi, out);
+    else if ((m & 0x03u) == 0x02u) bc7_mode_block<1, 2, 6, 0, 0, 6, 0, 0, 1, 3, 0>(lo, hi, out);
+    else if (m & 0x01u) bc7_mode_block<0, 3, 4, 0, 0, 4, 0, 1, 0, 3, 0>(lo, hi, out);
+    else if (m & 0x04u) bc7_mode_block<2, 3, 6, 0, 0, 5, 0, 0, 0, 2, 0>(lo, hi, out);
+    else if (m & 0x08u) bc7_mode_block<3, 2, 6, 0, 0, 7, 0, 1, 0, 2, 0>(lo, hi, out);
+    else if (m & 0x10u) bc7_mode_block<4, 1, 0, 2, 1, 5, 6, 0, 0, 2, 3>(lo, hi, out);
+    else if (m & 0x80u) bc7_mode_block<7, 2, 6, 0, 0, 5, 5, 1, 0, 2, 0>(lo, hi, out);
+    else {
         #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            x0[c] = (int)(((lo >> (7 + 14 * c)) & 0x7Fu) << 1) | p0;
-            x1[c] = (int)(((lo >> (14 + 14 * c)) & 0x7Fu) << 1) | p1;
-        }
-        const Lerp4 row(x0, x1);
-        #pragma unroll
-        for (int i = 0; i < 16; i++) out[i] = row.at(w4(i == 0 ? (int)((hi >> 1) & 7u) : (int)((hi >> (4 * i)) & 15u)));
-        return;
-    }
-    Bc7Fields F;
-    if (!bc7_parse(w, F)) {
-        for (int i = 0; i < 16; i++) out[i] = 0;
-        return;
-    }
-    for (int i = 0; i < 16; i++) {
-        const int s = F.subset[i];
-        int px[4];
-        for (int c = 0; c < 3; c++) px[c] = lerp64(F.ep[2 * s][c], F.ep[2 * s + 1][c], F.cw[i]);
-        px[3] = lerp64(F.ep[2 * s][3], F.ep[2 * s + 1][3], F.aw[i]);
-        if (F.rot) { int t = px[3]; px[3] = px[F.rot - 1]; px[F.rot - 1] = t; }
-        out[i] = pack_rgba(px[0], px[1], px[2], px[3]);
+        for (int i = 0; i < 16; i++) out[i] = 0u;
     }
 }
 
 // BC1 colour block; four_always: the BC3 colour half (zap_tex.h:1508-1517)
 ZTC_DEV void bc1_block(uint2 v, bool four_always, uint32_t out[16]) {
-    uint32_t c0 = v.x & 0xFFFFu, c1 = v.x >> 16;
-    int pal[4][3];
-    for (int k = 0; k < 2; k++) {
-        uint32_t c = k ? c1 : c0;
-        int R = (c >> 11) & 31, G = (c >> 5) & 63, B = c & 31;
-        pal[k][0] = (R << 3) | (R >> 2); pal[k][1] = (G << 2) | (G >> 4); pal[k][2] = (B << 3) | (B >> 2);
-    }
+    const uint32_t c0 = v.x & 0xFFFFu, c1 = v.x >> 16;
+    int a[3], b[3], p2[3], p3[3];
+    unpack565(c0, a[0], a[1], a[2]); unpack565(c1, b[0], b[1], b[2]);
     const bool four = four_always || c0 > c1;
+    #pragma unroll
     for (int c = 0; c < 3; c++) {
-        int a = pal[0][c], b = pal[1][c];
-        pal[2][c] = four ? (2 * a + b + 1) / 3 : (a + b + 1) / 2;
-        pal[3][c] = four ? (a + 2 * b + 1) / 3 : 0;
+        p2[c] = four ? (2 * a[c] + b[c] + 1) / 3 : (a[c] + b[c] + 1) / 2;
+        p3[c] = four ? (a[c] + 2 * b[c] + 1) / 3 : 0;
     }
+    const uint32_t q0 = pack_rgba(a[0], a[1], a[2], 255), q1 = pack_rgba(b[0], b[1], b[2], 255);
+    const uint32_t q2 = pack_rgba(p2[0], p2[1], p2[2], 255), q3 = pack_rgba(p3[0], p3[1], p3[2], four ? 255 : 0);
+    #pragma unroll
     for (int i = 0; i < 16; i++) {
-        int k = (int)((v.y >> (2 * i)) & 3u);
-        out[i] = pack_rgba(pal[k][0], pal[k][1], pal[k][2], (!four && k == 3) ? 0 : 255);
+        const bool b0 = (v.y >> (2 * i)) & 1u, b1 = (v.y >> (2 * i)) & 2u;
+        const uint32_t lo = b0 ? q1 : q0, hi = b0 ? q3 : q2;
+        out[i] = b1 ? hi : lo;
     }
 }
 
-// BC4 channel block (zap_tex.h:1519-1524)
-ZTC_DEV void bc4_block(uint2 v, uint8_t out[16]) {
-    int a0 = v.x & 0xFF, a1 = (v.x >> 8) & 0xFF, pal[8];
-    pal[0] = a0; pal[1] = a1;
-    if (a0 > a1) for (int i = 2; i < 8; i++) pal[i] = ((8 - i) * a0 + (i - 1) * a1 + 3) / 7;
-    else { for (int i = 2; i < 6; i++) pal[i] = ((6 - i) * a0 + (i - 1) * a1 + 2) / 5; pal[6] = 0; pal[7] = 255; }
-    uint64_t idx = (uint64_t)(v.x >> 16) | ((uint64_t)v.y << 16);
-    for (int i = 0; i < 16; i++) out[i] = (uint8_t)pal[(idx >> (3 * i)) & 7u];
+// bytes 0..7 of (lo, hi) picked by four 3-bit indices in nibbles
+ZTC_DEV uint32_t pick4(uint32_t lo, uint32_t hi, uint32_t nibbles) {
+#ifdef __CUDA_ARCH__
+    return __byte_perm(lo, hi, nibbles);
+#else
+    uint32_t r = 0;
+    for (int k = 0; k < 4; k++) {
+        const uint32_t j = (nibbles >> (4 * k)) & 7u;
+        r |= (((j < 4 ? lo : hi) >> (8 * (j & 3))) & 0xFFu) << (8 * k);
+    }
+    return r;
+#endif
+}
+// BC4 channel block (zap_tex.h:1519-1524): row r's four values in the bytes of out[r]
+ZTC_DEV void bc4_block(uint2 v, uint32_t out[4]) {
+    const int a0 = v.x & 0xFF, a1 = (v.x >> 8) & 0xFF;
+    const bool eight = a0 > a1;
+    uint32_t lo = (uint32_t)a0 | ((uint32_t)a1 << 8), hi = 0;
+    #pragma unroll
+    for (int i = 2; i < 8; i++) {
+        const int p = eight ? ((8 - i) * a0 + (i - 1) * a1 + 3) / 7 : i < 6 ? ((6 - i) * a0 + (i - 1) * a1 + 2) / 5 : i == 6 ? 0 : 255;
+        if (i < 4) lo |= (uint32_t)p << (8 * i); else hi |= (uint32_t)p << (8 * (i - 4));
+    }
+    const uint64_t idx = (uint64_t)(v.x >> 16) | ((uint64_t)v.y << 16);
+    #pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const uint32_t x = (uint32_t)(idx >> (12 * r));
+        out[r] = pick4(lo, hi, (x & 7u) | ((x & 0x38u) << 1) | ((x & 0x1C0u) << 2) | ((x & 0xE00u) << 3));
+    }
 }
 
-// one block of format fmt (0..4) to 16 RGBA8 texels (zap_tex.h:1526-1547)
 // A decoded 4x4 block of RGBA8 texels (px[i]: texel i, R in the low byte) into an image: each row of four texels
 // inside the image as one 16-byte store when vec (the image and its pitch 16-byte aligned), texels past the right
 // or bottom edge left out, a row the right edge cuts texel by texel (4-byte stores if aligned4, else bytes).
@@ -231,42 +320,63 @@ ZTC_DEV void store_block_rgba8(uint8_t *out, size_t stride, int w, int h, int bx
     }
 }
 
-ZTC_DEV void bcn_block(int fmt, const uint8_t *b, uint32_t out[16]) {
-    if (fmt == 0) { bc1_block(*(const uint2 *)b, false, out); return; }
-    if (fmt == 4) {
-        uint4 v = *(const uint4 *)b;
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        bc7_block(w, out);
-        return;
+// one block of format FMT (0..4) to 16 RGBA8 texels (zap_tex.h:1526-1547)
+template <int FMT>
+ZTC_DEV void bcn_block(const uint8_t *b, uint32_t out[16]) {
+    if (FMT == 0) {
+        bc1_block(ldg((const uint2 *)b), false, out);
+    } else if (FMT == 2) {
+        uint32_t r[4];
+        bc4_block(ldg((const uint2 *)b), r);
+        #pragma unroll
+        for (int i = 0; i < 16; i++) out[i] = chan(r[i >> 2], i & 3) | 0xFF000000u;
+    } else {
+        const uint4 v = ldg((const uint4 *)b);
+        if (FMT == 4) {
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            bc7_block(w, out);
+        } else if (FMT == 1) {
+            uint32_t a[4];
+            bc1_block(make_uint2(v.z, v.w), true, out);
+            bc4_block(make_uint2(v.x, v.y), a);
+            #pragma unroll
+            for (int i = 0; i < 16; i++) out[i] = (out[i] & 0x00FFFFFFu) | (chan(a[i >> 2], i & 3) << 24);
+        } else {
+            uint32_t r[4], g[4];
+            bc4_block(make_uint2(v.x, v.y), r);
+            bc4_block(make_uint2(v.z, v.w), g);
+            #pragma unroll
+            for (int i = 0; i < 16; i++) out[i] = chan(r[i >> 2], i & 3) | (chan(g[i >> 2], i & 3) << 8) | 0xFF000000u;
+        }
     }
-    uint8_t v0[16], v1[16];
-    if (fmt == 1) {
-        bc1_block(*(const uint2 *)(b + 8), true, out);
-        bc4_block(*(const uint2 *)b, v0);
-        for (int i = 0; i < 16; i++) out[i] = (out[i] & 0x00FFFFFFu) | ((uint32_t)v0[i] << 24);
-        return;
-    }
-    bc4_block(*(const uint2 *)b, v0);
-    if (fmt == 3) bc4_block(*(const uint2 *)(b + 8), v1);
-    else for (int i = 0; i < 16; i++) v1[i] = 0;
-    for (int i = 0; i < 16; i++) out[i] = pack_rgba(v0[i], v1[i], 0, 255);
 }
 
-// BC6H mode 11 to half bits, alpha 1.0 (zap_tex.h:933-943); other modes decode to 0
-ZTC_DEV void bc6h_block(const uint32_t w[4], uint16_t out[16][4]) {
-    for (int i = 0; i < 16; i++) out[i][0] = out[i][1] = out[i][2] = out[i][3] = 0;
-    if (get_bits128(w, 0, 5) != 3u) return;
-    int e[2][3];
-    for (int k = 0; k < 2; k++)
-        for (int c = 0; c < 3; c++) {
-            int q = (int)get_bits128(w, 5 + 10 * (3 * k + c), 10);
-            e[k][c] = q == 0 ? 0 : q == 1023 ? 0xFFFF : ((q << 16) + 0x8000) >> 10;
+// BC6H mode 11 to half bits, alpha 1.0 (zap_tex.h:933-943): texel i in out[2 i] (R, G) and out[2 i + 1] (B, A); other
+// modes decode to 0. A channel's lerp is affine in the weight: 64 a + 32 + (b - a) w, never negative.
+ZTC_DEV void bc6h_block(const uint32_t w[4], uint32_t out[32]) {
+    const uint64_t lo = w[0] | ((uint64_t)w[1] << 32), hi = w[2] | ((uint64_t)w[3] << 32);
+    const bool ok = (w[0] & 31u) == 3u;
+    int base[3], slope[3];
+    #pragma unroll
+    for (int c = 0; c < 3; c++) {
+        int e[2];
+        #pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int q = (int)field64(lo, hi, 5 + 10 * (3 * k + c), 10);
+            e[k] = q == 0 ? 0 : q == 1023 ? 0xFFFF : ((q << 16) + 0x8000) >> 10;
         }
+        base[c] = 64 * e[0] + 32;
+        slope[c] = e[1] - e[0];
+    }
+    const uint64_t idx = open_bit(field64(lo, hi, 65, 63), 3);
+    #pragma unroll
     for (int i = 0; i < 16; i++) {
-        int idx = i == 0 ? (int)get_bits128(w, 65, 3) : (int)get_bits128(w, 68 + 4 * (i - 1), 4);
-        int wt = w4(idx);
-        for (int c = 0; c < 3; c++) out[i][c] = (uint16_t)((lerp64(e[0][c], e[1][c], wt) * 31) >> 6);
-        out[i][3] = 0x3C00;
+        const int wt = weight_of<4>((uint32_t)(idx >> (4 * i)) & 15u);
+        uint32_t h[3];
+        #pragma unroll
+        for (int c = 0; c < 3; c++) h[c] = ((uint32_t)((base[c] + slope[c] * wt) >> 6) * 31u) >> 6;
+        out[2 * i] = ok ? h[0] | (h[1] << 16) : 0u;
+        out[2 * i + 1] = ok ? h[2] | 0x3C000000u : 0u;
     }
 }
 
