@@ -52,3 +52,33 @@ def test_channel_blocks(cuda_lib, oracle, fmt, channels, size):
         t = torch.from_numpy(img[..., :channels].copy()).cuda()[:, x0:]
         if sub.shape[1]:
             assert np.array_equal(zap_b200.bc_encode_dev(t, fmt).cpu().numpy(), oracle.bc_encode(sub, fmt)), (fmt, size, x0)
+
+
+def test_scratch_pool_across_streams_threads_and_capture(cuda_lib, oracle):
+    """Scratch from the context's pool: calls on several streams and threads at once, and a captured call replayed."""
+    import threading
+    imgs = [_image(64 + 16 * k, 80, 40 + k) for k in range(4)]
+    want = [oracle.bc_encode(i, zap_b200.BC7) for i in imgs]
+    texs = [torch.from_numpy(i).cuda() for i in imgs]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(k):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            outs = [zap_b200.bc_encode_dev(texs[k], zap_b200.BC7) for _ in range(8)]
+        s.synchronize()
+        bad.extend(k for o in outs if not np.array_equal(o.cpu().numpy(), want[k]))
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
+    out = torch.zeros(want[0].size, dtype=torch.uint8, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        zap_b200.bc_encode_dev(texs[0], zap_b200.BC7, out=out)
+    for _ in range(3):
+        out.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy(), want[0])

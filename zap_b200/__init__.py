@@ -51,6 +51,12 @@ def bc_size(w, h, fmt):
     return int(load().zap_tex_cuda_bc_size(w, h, fmt))
 
 
+def _empty_blocks(t, w, h, fmt):
+    """A device buffer for the encoded blocks of t: bc_size(w, h, fmt) bytes, without the library call."""
+    import torch
+    return t.new_empty(((w + 3) >> 2) * ((h + 3) >> 2) * (8 if fmt in (BC1, BC4) else 16), dtype=torch.uint8)
+
+
 def mip_levels(w, h):
     return int(load().zap_tex_cuda_mip_levels(w, h))
 
@@ -112,15 +118,18 @@ def mip_next_f(rgba, ctx=None):
 
 # ---------------------------------------------------------------- device memory (torch CUDA tensors)
 def _stream(stream):
+    """The stream's handle (the current device's current stream when none is given)."""
+    if stream is not None:
+        return stream.cuda_stream
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # the handle alone: no Stream object per call
 
 
 def _dev_img(t, channels=(4,)):
-    if not t.is_cuda or t.dim() != 3 or t.shape[2] not in channels or t.stride(2) != 1 or t.stride(1) != t.shape[2]:
-        raise ValueError(f"expected an HxWxC CUDA tensor with C in {channels} and packed rows, got {tuple(t.shape)}")
-    return t.shape[1], t.shape[0], t.stride(0)
+    shape, stride = t.shape, t.stride()
+    if not t.is_cuda or len(shape) != 3 or shape[2] not in channels or stride[2] != 1 or stride[1] != shape[2]:
+        raise ValueError(f"expected an HxWxC CUDA tensor with C in {channels} and packed rows, got {tuple(shape)}")
+    return shape[1], shape[0], stride[0]
 
 
 def bc_encode_dev(t, fmt, out=None, stream=None, ctx=None):
@@ -130,7 +139,7 @@ def bc_encode_dev(t, fmt, out=None, stream=None, ctx=None):
         raise ValueError("expected uint8")
     w, h, stride = _dev_img(t, (1, 2, 4))
     if out is None:
-        out = torch.empty(bc_size(w, h, fmt), dtype=torch.uint8, device=t.device)
+        out = _empty_blocks(t, w, h, fmt)
     check(load().zap_tex_cuda_bc_encode_u8_dev(ctx, t.data_ptr(), t.shape[2], w, h, stride, fmt, out.data_ptr(), _stream(stream)),
           "bc_encode_dev")
     return out
@@ -142,7 +151,7 @@ def bc_encode_rdo_dev(t, fmt, rdo, band_rows=0, out=None, stream=None, ctx=None)
     import torch
     w, h, stride = _dev_img(t, (4,))
     if out is None:
-        out = torch.empty(bc_size(w, h, fmt), dtype=torch.uint8, device=t.device)
+        out = _empty_blocks(t, w, h, fmt)
     check(load().zap_tex_cuda_bc_encode_rdo_dev(ctx, t.data_ptr(), w, h, stride, fmt, float(rdo), int(band_rows), out.data_ptr(),
                                                 _stream(stream)), "bc_encode_rdo_dev")
     return out
@@ -162,7 +171,7 @@ def bc6h_encode_dev(t, out=None, stream=None, ctx=None):
     else:
         raise ValueError("expected float32 RGBA or float16 RGB(A)")
     if out is None:
-        out = torch.empty(bc_size(w, h, BC6H), dtype=torch.uint8, device=t.device)
+        out = _empty_blocks(t, w, h, BC6H)
     lib = load()
     if t.dtype == torch.float32:
         st = lib.zap_tex_cuda_bc6h_encode_dev(ctx, t.data_ptr(), w, h, stride, out.data_ptr(), _stream(stream))
@@ -239,7 +248,7 @@ def bc_encode_split_dev(t, fmt, out=None, stream=None, ctx=None):
     import torch
     w, h, stride = _dev_img(t, (4,))
     if out is None:
-        out = torch.empty(bc_size(w, h, fmt), dtype=torch.uint8, device=t.device)
+        out = _empty_blocks(t, w, h, fmt)
     check(load().zap_tex_cuda_bc_encode_split_dev(ctx, t.data_ptr(), w, h, stride, fmt, out.data_ptr(), _stream(stream)),
           "bc_encode_split_dev")
     return out
@@ -450,6 +459,6 @@ def mip_chain_dev(t, srgb, stream=None, ctx=None):
     levels, off = [], 0
     while w > 1 or h > 1:
         w, h = max(1, w // 2), max(1, h // 2)
-        levels.append(buf[off:off + w * h * 4].view(h, w, 4))
+        levels.append(buf.as_strided((h, w, 4), (4 * w, 4, 1), off))
         off += w * h * 4
     return levels

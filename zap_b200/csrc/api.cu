@@ -99,8 +99,15 @@ struct zap_tex_cuda_ctx {
     size_t d_out_cap = 0;
     void *d_scratch[2] = {nullptr, nullptr};
     size_t d_scratch_cap[2] = {0, 0};
+    // Stream-ordered scratch of the context's calls. A pool of its own that keeps up to kPoolKeep bytes across
+    // synchronisations: the device's default pool gives everything back at each one, so every call after a wait
+    // mapped its scratch anew (0.45 to 4 ms; a 64x64 BC7 call 0.5 ms instead of 0.05). It takes calls from any thread and
+    // stream, and goes with the context.
+    cudaMemPool_t pool = nullptr;
     bool owned_default = false;
 };
+// what a pool keeps: the scratch of calls up to 16384x8192 (8 bytes a block); larger scratch is given back
+constexpr uint64_t kPoolKeep = 64ull << 20;
 
 namespace {
 
@@ -169,6 +176,13 @@ int create_ctx(int device, zap_tex_cuda_ctx **out) {
             zap_tex_cuda_destroy(c);
             return cuda_fail(cudaErrorUnknown, "event creation");
         }
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = kPoolKeep;
+    if (cudaMemPoolCreate(&c->pool, &props) != cudaSuccess) { cudaGetLastError(); c->pool = nullptr; }  // the default pool serves
+    else cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
     *out = c;
     return ZTC_OK;
 }
@@ -309,12 +323,11 @@ int dev_encode(zap_tex_cuda_ctx *ctx, int fmt, const ztc::SrcU8 &s8, const ztc::
     const size_t bs = fmt == ZTC_BC6H || fmt == ZTC_ASTC4X4 ? 16 : block_bytes(fmt);
     const size_t scr = scratch_for(fmt, (size_t)bw * rows);
     void *scratch = nullptr;
-    if (scr) ZTC_CHECK(ztc_malloc_async(&scratch, scr, s), "cudaMallocAsync(scratch)");
+    if (scr) ZTC_CHECK(ztc_malloc_async(&scratch, scr, s, ctx), "cudaMallocAsync(scratch)");
     int st = ZTC_OK;
     for (int y = 0; y < bh && !st; y += rows)  // launches on one stream, so they share the scratch in turn
         st = launch_encode(fmt, s8, sh, y, rows < bh - y ? rows : bh - y, (uint8_t *)out + (size_t)y * bw * bs, scratch, s);
     if (scratch) cudaFreeAsync(scratch, s);
-    (void)ctx;
     return st;
 }
 
@@ -323,7 +336,7 @@ int dev_encode(zap_tex_cuda_ctx *ctx, int fmt, const ztc::SrcU8 &s8, const ztc::
 int rdo_encode(zap_tex_cuda_ctx *ctx, int fmt, const ztc::SrcU8 &s8, int w, int h, float lambda, int band_rows, void *out, cudaStream_t s) {
     int st = dev_encode(ctx, fmt, s8, nullptr, w, h, out, s);
     if (st) return st;
-    ZTC_CHECK(ztc_launch_rdo(fmt, s8, (uint8_t *)out, lambda, band_rows, s), "rdo launch");
+    ZTC_CHECK(ztc_launch_rdo(fmt, s8, (uint8_t *)out, lambda, band_rows, ctx, s), "rdo launch");
     return ZTC_OK;
 }
 
@@ -361,9 +374,10 @@ cudaError_t ztc_malloc(void **p, size_t n) {
     if (alloc_fault()) { *p = nullptr; return cudaErrorMemoryAllocation; }
     return cudaMalloc(p, n);
 }
-cudaError_t ztc_malloc_async(void **p, size_t n, cudaStream_t s) {
+cudaError_t ztc_malloc_async(void **p, size_t n, cudaStream_t s, zap_tex_cuda_ctx *ctx) {
     if (alloc_fault()) { *p = nullptr; return cudaErrorMemoryAllocation; }
-    return cudaMallocAsync(p, n, s);
+    if (!ctx && resolve(ctx) != ZTC_OK) { *p = nullptr; return cudaErrorInvalidDevice; }
+    return ctx->pool ? cudaMallocFromPoolAsync(p, n, ctx->pool, s) : cudaMallocAsync(p, n, s);
 }
 cudaError_t ztc_malloc_host(void **p, size_t n) {
     if (alloc_fault()) { *p = nullptr; return cudaErrorMemoryAllocation; }
@@ -484,6 +498,7 @@ int zap_tex_cuda_destroy(zap_tex_cuda_ctx *c) {
     for (int k = 0; k < kStreams; k++) if (c->stream[k]) { cudaStreamSynchronize(c->stream[k]); cudaStreamDestroy(c->stream[k]); }
     if (c->ev_in) cudaEventDestroy(c->ev_in);
     for (int k = 0; k <= kOutLag; k++) if (c->ev_enc[k]) cudaEventDestroy(c->ev_enc[k]);
+    if (c->pool) cudaMemPoolDestroy(c->pool);  // memory still in use by queued calls goes when they end
     cudaFree(c->d_in); cudaFree(c->d_out); cudaFree(c->d_scratch[0]); cudaFree(c->d_scratch[1]);
     if (c->owned_default) {
         std::lock_guard<std::mutex> g(g_lock);
@@ -498,13 +513,13 @@ int zap_tex_cuda_reserve(zap_tex_cuda_ctx *ctx, size_t bytes) {
     ZTC_NVTX();
     int st = resolve(ctx);
     if (st) return st;
-    // _dev calls draw scratch from the device's default memory pool: keep that much resident across frees
-    cudaMemPool_t pool;
-    ZTC_CHECK(cudaDeviceGetDefaultMemPool(&pool, ctx->device), "cudaDeviceGetDefaultMemPool");
-    uint64_t keep = bytes;
+    // _dev calls draw scratch from the context's memory pool: keep that much resident across frees
+    cudaMemPool_t pool = ctx->pool;
+    if (!pool) ZTC_CHECK(cudaDeviceGetDefaultMemPool(&pool, ctx->device), "cudaDeviceGetDefaultMemPool");
+    uint64_t keep = ctx->pool && bytes < kPoolKeep ? kPoolKeep : bytes;
     ZTC_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
     void *p = nullptr;
-    ZTC_CHECK(ztc_malloc_async(&p, bytes ? bytes : 1, ctx->stream[0]), "cudaMallocAsync(reserve)");
+    ZTC_CHECK(ztc_malloc_async(&p, bytes ? bytes : 1, ctx->stream[0], ctx), "cudaMallocAsync(reserve)");
     ZTC_CHECK(cudaFreeAsync(p, ctx->stream[0]), "cudaFreeAsync(reserve)");
     ZTC_CHECK(cudaStreamSynchronize(ctx->stream[0]), "reserve");
     return ZTC_OK;
@@ -697,7 +712,7 @@ int zap_tex_cuda_bc_encode_split_dev(zap_tex_cuda_ctx *ctx, const uint8_t *rgba,
         return ZTC_OK;
     }
     void *scratch = nullptr;
-    ZTC_CHECK(ztc_malloc_async(&scratch, ztc::bc7_scratch_bytes((size_t)bw * bh), s), "cudaMallocAsync(scratch)");
+    ZTC_CHECK(ztc_malloc_async(&scratch, ztc::bc7_scratch_bytes((size_t)bw * bh), s, ctx), "cudaMallocAsync(scratch)");
     cudaError_t e = ztc_launch_bc7_to(s8, 0, bh, planes, 0, scratch, s);
     cudaFreeAsync(scratch, s);
     if (e != cudaSuccess) return cuda_fail(e, "kernel launch");

@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) rdo_sub_chain_kernel(SrcU8 src
 
 // RDO pass over an image whose base encodings `out` holds (raster blocks): one chain per band of band_rows block
 // rows (band_rows >= the block-row count: one chain, the reference's single call). lambda: finite, > 0.
-cudaError_t ztc_launch_rdo(int fmt, const ztc::SrcU8 &src, uint8_t *out, float lambda, int band_rows, cudaStream_t stream) {
+cudaError_t ztc_launch_rdo(int fmt, const ztc::SrcU8 &src, uint8_t *out, float lambda, int band_rows, zap_tex_cuda_ctx *ctx, cudaStream_t stream) {
     const int bw = (src.w + 3) / 4, nby = (src.h + 3) / 4;
     if (band_rows <= 0 || band_rows > nby) band_rows = nby;
     const int chains = (nby + band_rows - 1) / band_rows;
@@ -670,7 +670,7 @@ cudaError_t ztc_launch_rdo(int fmt, const ztc::SrcU8 &src, uint8_t *out, float l
     if (fmt == ZTC_FMT_BC7) {
         const int nblocks = bw * nby;
         uint32_t *dec = nullptr;
-        cudaError_t e = ztc_malloc_async((void **)&dec, (size_t)nblocks * 64, stream);
+        cudaError_t e = ztc_malloc_async((void **)&dec, (size_t)nblocks * 64, stream, ctx);
         if (e != cudaSuccess) return e;
         ztc::bc7_decode_bases_kernel<<<(nblocks + 127) / 128, 128, 0, stream>>>(out, nblocks, (uint4 *)dec);
         constexpr int L = ZTC_RDO_BC7_LANES;

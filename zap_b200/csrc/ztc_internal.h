@@ -120,13 +120,13 @@ void srgb_tables_host(SrgbTables &t);
 // ones fail (zap_tex_cuda_debug_fail_allocations) and check that each entry point reports ZTC_ERR_NO_MEMORY and the
 // library keeps working afterwards.
 cudaError_t ztc_malloc(void **p, size_t n);
-cudaError_t ztc_malloc_async(void **p, size_t n, cudaStream_t s);
+struct zap_tex_cuda_ctx;
+cudaError_t ztc_malloc_async(void **p, size_t n, cudaStream_t s, zap_tex_cuda_ctx *ctx);  // from ctx's pool (NULL: the default context's)
 cudaError_t ztc_malloc_host(void **p, size_t n);
 
 // records the calling thread's error message (zap_tex_cuda_last_error) and returns status
 int ztc_set_error(int status, const char *msg);
 // makes ctx's device current (NULL: the current device's default context) with its tables uploaded
-struct zap_tex_cuda_ctx;
 int ztc_ctx_activate(zap_tex_cuda_ctx *ctx);
 
 cudaError_t ztc_launch_bcn(int fmt, const ztc::SrcU8 &src, int by0, int nby, uint8_t *out, cudaStream_t stream);
@@ -139,7 +139,7 @@ cudaError_t ztc_launch_bc7_to(const ztc::SrcU8 &src, int by0, int nby, const ztc
 // RDO (lambda > 0) over base encodings already in `out`, in place: one chain per band_rows block rows (0: one)
 // SMs of the current device (cached per device)
 int ztc_sm_count();
-cudaError_t ztc_launch_rdo(int fmt, const ztc::SrcU8 &src, uint8_t *out, float lambda, int band_rows, cudaStream_t stream);
+cudaError_t ztc_launch_rdo(int fmt, const ztc::SrcU8 &src, uint8_t *out, float lambda, int band_rows, zap_tex_cuda_ctx *ctx, cudaStream_t stream);
 // split (to_planes = 1) or merge n bytes of BC1..BC7 data, device to device (zap_tex.h:1549-1571)
 cudaError_t ztc_launch_bc_regroup(const uint8_t *in, uint8_t *out, size_t n, int fmt, int to_planes, cudaStream_t stream);
 cudaError_t ztc_launch_bc6h(const ztc::SrcHdr &src, int by0, int nby, uint8_t *out, cudaStream_t stream);
