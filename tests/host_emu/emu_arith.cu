@@ -52,3 +52,22 @@ EMU uint64_t emu_bc4_distance_mismatches(int ulps) {
             }
     return bad;
 }
+
+// floats v in [-512, 768] with bit patterns in [lo, hi) (either sign) for which quant8_pbits differs from quant_pbit
+EMU uint64_t emu_quant8_mismatches(uint64_t lo, uint64_t hi) {
+    uint64_t bad = 0;
+    for (uint64_t b = lo; b < hi; b++) {
+        const float v[4] = {u_as_f((uint32_t)b), 0.0f, 0.0f, 0.0f};
+        if (!(v[0] >= -512.0f && v[0] <= 768.0f)) continue;
+        uint32_t k[2][4];
+        int err[2];
+        quant8_pbits<1>(v, k, err);
+        for (int p = 0; p < 2; p++) {
+            int q[4], x8[4];
+            const int e = quant_pbit<1>(v, 8, p, q, x8);
+            const int got = (int)(k[p][0] & 127u);
+            bad += e != err[p] || q[0] != got || x8[0] != 2 * got + p;
+        }
+    }
+    return bad;
+}

@@ -50,3 +50,15 @@ def test_srgb_one_word_search_equals_binary_search(emu):
 def test_bc4_distance_equals_palette_scan(emu, ulps):
     """Every endpoint pair and every level within the insets around it, at a reciprocal a few ulp off too."""
     assert emu.emu_bc4_distance_mismatches(ulps) == 0
+
+
+def test_quant8_equals_three_candidate_search(emu):
+    """The mode-6 endpoint quantiser for every float in [-512, 768] and both p-bits."""
+    emu.emu_quant8_mismatches.argtypes = [C.c_uint64, C.c_uint64]
+    emu.emu_quant8_mismatches.restype = C.c_uint64
+    chunks = []
+    for base, top in ((0, _bits(768.0) + 1), (0x80000000, 0x80000000 + _bits(512.0) + 1)):
+        step = (top - base + 63) // 64
+        chunks += [(base + k * step, min(top, base + (k + 1) * step)) for k in range(64)]
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as ex:
+        assert sum(ex.map(lambda c: emu.emu_quant8_mismatches(*c), chunks)) == 0

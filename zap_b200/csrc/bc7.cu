@@ -56,9 +56,11 @@ ZTC_DEV int palette_fit(TexRef ts, uint32_t mask, const int x0[4], const int x1[
     for (int i = 0; i < 16; i++) {
         if (!((mask >> i) & 1u)) continue;
         const uint32_t p = ts[i] & cm;
-        int m = A[0] - 2 * NP * (int)dot4(p, pal[0]);
+        int m = (int)0x80000000;  // minus the least key: shifts and three-way maxima measured 1 % under multiply-adds and minima
         #pragma unroll
-        for (int j = 1; j < NP; j++) m = min(m, A[j] - 2 * NP * (int)dot4(p, pal[j]));
+        for (int j = 0; j < NP; j += 2)
+            m = max3i(m, (int)(dot4(p, pal[j]) << (IB + 1)) - A[j], (int)(dot4(p, pal[j + 1]) << (IB + 1)) - A[j + 1]);
+        m = -m;
         err += (m >> IB) + (int)dot4(p, p);
         bits |= (uint64_t)(m & (NP - 1)) << (4 * i);
     }
@@ -69,6 +71,19 @@ ZTC_DEV int palette_fit(TexRef ts, uint32_t mask, const int x0[4], const int x1[
 // float endpoints -> best p-bits and quantised endpoints q (x0, x1: expanded to 8 bits) (zap_tex.h:466-486)
 template <int NC>
 ZTC_DEV void subset_quant(int n, bool shared_p, const float lo[4], const float hi[4], int q[2][4], int pb[2], int x0[4], int x1[4]) {
+    if (n == 8 && !shared_p) {  // mode 6: the two endpoints' p-bits are independent, p = 0 on ties
+        uint32_t kl[2][4], kh[2][4];
+        int el[2], eh[2];
+        quant8_pbits<NC>(lo, kl, el); quant8_pbits<NC>(hi, kh, eh);
+        pb[0] = el[1] < el[0]; pb[1] = eh[1] < eh[0];
+        #pragma unroll
+        for (int c = 0; c < 4; c++) {
+            q[0][c] = c < NC ? (int)((pb[0] ? kl[1][c] : kl[0][c]) & 127u) : 0;
+            q[1][c] = c < NC ? (int)((pb[1] ? kh[1][c] : kh[0][c]) & 127u) : 0;
+            x0[c] = 2 * q[0][c] + pb[0]; x1[c] = 2 * q[1][c] + pb[1];
+        }
+        return;
+    }
     int ql[2][4], qh[2][4], xl[2][4], xh[2][4], el[2], eh[2];
     #pragma unroll
     for (int p = 0; p < 2; p++) { el[p] = quant_pbit<NC>(lo, n, p, ql[p], xl[p]); eh[p] = quant_pbit<NC>(hi, n, p, qh[p], xh[p]); }
@@ -111,18 +126,31 @@ ZTC_DEV int subset_passes(TexRef ts, uint32_t mask, int n, bool shared_p, float 
     for (int it = first; it < last; it++) {
         if (it > 0) {
             if (err <= 0) return err;
-            float aa = 0.0f, ab = 0.0f, bb = 0.0f, sa[NC], sb[NC];
+            // Every term and partial sum of the reference's float sums is exact: w = k / 64 for an integer k in 0..64, so u u,
+            // u w, w w are multiples of 2^-12 with sums at most 16, and u x, w x multiples of 2^-6 with sums below 2^12.
+            // So they are integer dot products over the texels, a byte a texel, scaled (texels outside the subset have
+            // index 0 and weight 0): with K the weights, sum (64 - K)^2 = 4096 n - 128 sum K + sum K^2, and so on.
+            uint32_t W1 = 0u, W2 = 0u, SX[NC], SB[NC];
             #pragma unroll
-            for (int c = 0; c < NC; c++) { sa[c] = 0.0f; sb[c] = 0.0f; }
-            #pragma unroll 1
-            for (int i = 0; i < 16; i++) {
-                if (!((mask >> i) & 1u)) continue;
-                float w = small_u2f((uint32_t)wbits(IB, (int)((idx >> (4 * i)) & 15u))) / 64.0f, u = 1.0f - w;
-                aa = aa + u * u; ab = ab + u * w; bb = bb + w * w;
-                const uint32_t x = ts[i];
+            for (int c = 0; c < NC; c++) { SX[c] = 0u; SB[c] = 0u; }
+            #pragma unroll
+            for (int r = 0; r < 4; r++) {
+                uint32_t j = (uint32_t)(idx >> (16 * r)) & 0xFFFFu, x[4];
+                j = (j | (j << 8)) & 0x00FF00FFu;
+                j = (j | (j << 4)) & 0x0F0F0F0Fu;  // the row's four indices, a byte each
+                const uint32_t K = IB == 4 ? 4u * j + (((j + 0x02020202u) >> 2) & 0x07070707u) : 9u * j + ((j >> 2) & 0x01010101u);
+                const uint32_t ones = mask == 0xFFFFu ? 0x01010101u : (((mask >> (4 * r)) & 15u) * 0x00204081u) & 0x01010101u;
+                by_channel(ts[4 * r], ts[4 * r + 1], ts[4 * r + 2], ts[4 * r + 3], x);
+                W1 = dot4_add(K, 0x01010101u, W1); W2 = dot4_add(K, K, W2);
                 #pragma unroll
-                for (int c = 0; c < NC; c++) { float xc = small_u2f(chan(x, c)); sa[c] = sa[c] + u * xc; sb[c] = sb[c] + w * xc; }
+                for (int c = 0; c < NC; c++) { SX[c] = dot4_add(x[c], ones, SX[c]); SB[c] = dot4_add(x[c], K, SB[c]); }
             }
+            const uint32_t n16 = mask == 0xFFFFu ? 16u : (uint32_t)popc(mask);
+            const float aa = small_u2f(4096u * n16 - 128u * W1 + W2) * (1.0f / 4096.0f), ab = small_u2f(64u * W1 - W2) * (1.0f / 4096.0f);
+            const float bb = small_u2f(W2) * (1.0f / 4096.0f);
+            float sa[NC], sb[NC];
+            #pragma unroll
+            for (int c = 0; c < NC; c++) { sa[c] = small_u2f(64u * SX[c] - SB[c]) * (1.0f / 64.0f); sb[c] = small_u2f(SB[c]) * (1.0f / 64.0f); }
             float det = aa * bb - ab * ab;
             if (det < 1e-6f && det > -1e-6f) return err;
             #pragma unroll

@@ -215,6 +215,81 @@ ZTC_DEV int quant_pbit(const float v[4], int n, int p, int q[4], int x8[4]) {
     return err;
 }
 
+// ceil(a - b) + 1.5 * 2^23 as a float, for a - b well inside +-2^22: both sums round up, and a difference that rounds up
+// stays at or below the next integer
+ZTC_DEV float ceil_sub_magic(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fadd_ru(__fadd_ru(a, -b), 12582912.0f);
+#else
+    return (float)std::ceil((double)a - (double)b) + 12582912.0f;
+#endif
+}
+// 2^23 + floor(v) for 0 <= v < 2^23, as bits
+ZTC_DEV uint32_t floor_bits(float v) {
+#ifdef __CUDA_ARCH__
+    return __float_as_uint(__fadd_rz(v, 8388608.0f));
+#else
+    return f_as_u(std::floor(v) + 8388608.0f);
+#endif
+}
+// quant_pbit at 8 bits for both p-bits at once, by rule instead of by trying three candidates: the value of parity p
+// nearest to v, the lower one on a tie (two candidates' truncated squares tie only where both are 1 away, and the
+// lower is tried first), within [p, 254 + p]. k[p][c] holds the stored 7-bit value in its low bits; err[p] the sum of
+// the truncated squares. About 19 operations a channel instead of about 90; equal to quant_pbit for every float in
+// the domain given there (the host test checks all of them).
+template <int NC>
+ZTC_DEV void quant8_pbits(const float v[4], uint32_t k[2][4], int err[2]) {
+    uint32_t e0 = 0u, e1 = 0u;
+    #pragma unroll
+    for (int c = 0; c < NC; c++) {
+        const float h = v[c] * 0.5f;
+        const float r0 = fminf(fmaxf(ceil_sub_magic(h, 0.5f), 12582912.0f), 12583039.0f);  // + 0 .. + 127
+        const float r1 = fminf(fmaxf(ceil_sub_magic(h, 1.0f), 12582912.0f), 12583039.0f);
+        const float d0 = fma_rn(r0 - 12582912.0f, 2.0f, -v[c]), d1 = fma_rn(r1 - 12582912.0f, 2.0f, 1.0f) - v[c];
+        e0 += floor_bits(d0 * d0) - 0x4B000000u;
+        e1 += floor_bits(d1 * d1) - 0x4B000000u;
+        k[0][c] = f_as_u(r0); k[1][c] = f_as_u(r1);
+    }
+    err[0] = (int)e0; err[1] = (int)e1;
+}
+
+// four texels' channels, a byte per texel: word c of x holds channel c of t0..t3
+ZTC_DEV void by_channel(uint32_t t0, uint32_t t1, uint32_t t2, uint32_t t3, uint32_t x[4]) {
+#ifdef __CUDA_ARCH__
+    const uint32_t a = __byte_perm(t0, t1, 0x5140u), b = __byte_perm(t2, t3, 0x5140u);
+    const uint32_t c = __byte_perm(t0, t1, 0x7362u), d = __byte_perm(t2, t3, 0x7362u);
+    x[0] = __byte_perm(a, b, 0x5410u); x[1] = __byte_perm(a, b, 0x7632u);
+    x[2] = __byte_perm(c, d, 0x5410u); x[3] = __byte_perm(c, d, 0x7632u);
+#else
+    for (int k = 0; k < 4; k++) {
+        const int s = 8 * k;
+        x[k] = ((t0 >> s) & 0xFFu) | (((t1 >> s) & 0xFFu) << 8) | (((t2 >> s) & 0xFFu) << 16) | (((t3 >> s) & 0xFFu) << 24);
+    }
+#endif
+}
+#ifdef __CUDA_ARCH__
+ZTC_DEV int max3i(int a, int b, int c) { return __vimax3_s32(a, b, c); }
+#else
+inline int max3i(int a, int b, int c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
+#endif
+ZTC_DEV uint32_t dot4_add(uint32_t a, uint32_t b, uint32_t c) {
+#ifdef __CUDA_ARCH__
+    return __dp4a(a, b, c);
+#else
+    return dot4(a, b) + c;
+#endif
+}
+// channel c of texel x as the float 32768 + value; less 32768 + m for a multiple m of 2^-8 it is value - m, exactly
+ZTC_DEV float texel_at_2p15(uint32_t x, int c) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(__byte_perm(x, 0x47000000u, 0x7404u | (uint32_t)(c << 4)));
+#else
+    return u_as_f(0x47000000u | (((x >> (8 * c)) & 0xFFu) << 8));
+#endif
+}
+// an integer in (-2^22, 2^22) as a float
+ZTC_DEV float small_i2f(int n) { return u_as_f(0x4B400000u + (uint32_t)n) - 12582912.0f; }
+
 // 565 endpoint -> 8-bit RGB by bit replication (zap_tex.h:41-44)
 ZTC_DEV void unpack565(uint32_t c, int &r, int &g, int &b) {
     int R = (c >> 11) & 31, G = (c >> 5) & 63, B = c & 31;

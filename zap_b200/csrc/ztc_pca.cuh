@@ -33,22 +33,66 @@ ZTC_DEV float pca_u2f(uint32_t n) { return BITS ? small_u2f(n) : (float)n; }
 // (the same operations in the same order, in less code), UNROLL 16 unrolls them; U2F_BITS: pca_u2f's form
 template <int NC, int UNROLL = 16, bool U2F_BITS = true, typename Tex>
 ZTC_DEV void pca_endpoints(const Tex &t, uint32_t mask, float lo[4], float hi[4]) {
-    const float cnt = pca_u2f<U2F_BITS>((uint32_t)popc(mask)), cnti = 1.0f / cnt;
-    const bool whole = mask == 0xFFFFu;  // a compile-time constant for whole-block calls: x / 16 is a multiply there
-    float mu[NC];
+    const bool whole = mask == 0xFFFFu;  // a compile-time constant for whole-block calls
+    float mu[NC], C[NC][NC];
     if (whole) {
-        // every term x / 16 and every partial sum of the mean is exact (a multiple of 1/16 below 256), so the
-        // float sum is the channel's integer sum / 16; the four sums in two words of 16-bit fields
-        uint32_t s02 = 0, s13 = 0;
-        for_texels<UNROLL>([&](int i) {
-            const uint32_t x = t[i];
-            s02 += x & 0x00FF00FFu;
-            s13 += (x >> 8) & 0x00FF00FFu;
-        });
-        const uint32_t S[4] = {s02 & 0xFFFFu, s13 & 0xFFFFu, s02 >> 16, s13 >> 16};
+        // The reference's mean sums x / 16 and its covariance d_a d_b over the texels, d = x - mean. d is a multiple of 1/16 below
+        // 2^8, so each product is exact (24 bits), and so is every partial sum while it stays below 2^16; they all do
+        // when each channel's sum of d^2 is below 2^16. Then the floats are the integer sums 16 sum x_a x_b - S_a S_b
+        // over 16, whatever their order: 14 dot products per four texels instead of 20 float operations and 8
+        // conversions per texel. Blocks with a wider channel (Q below 2^20 fails) take the sums as the reference does.
+        uint32_t S[NC], Q[NC][NC];
         #pragma unroll
-        for (int c = 0; c < NC; c++) mu[c] = pca_u2f<U2F_BITS>(S[c]) / 16.0f;
+        for (int a = 0; a < NC; a++) {
+            S[a] = 0u;
+            #pragma unroll
+            for (int b = a; b < NC; b++) Q[a][b] = 0u;
+        }
+        const auto row = [&](int r) {
+            uint32_t x[4];
+            by_channel(t[4 * r], t[4 * r + 1], t[4 * r + 2], t[4 * r + 3], x);
+            #pragma unroll
+            for (int a = 0; a < NC; a++) {
+                S[a] = dot4_add(x[a], 0x01010101u, S[a]);
+                #pragma unroll
+                for (int b = a; b < NC; b++) Q[a][b] = dot4_add(x[a], x[b], Q[a][b]);
+            }
+        };
+        if (UNROLL == 1) {
+            #pragma unroll 1
+            for (int r = 0; r < 4; r++) row(r);
+        } else {
+            #pragma unroll
+            for (int r = 0; r < 4; r++) row(r);
+        }
+        bool exact = true;
+        #pragma unroll
+        for (int a = 0; a < NC; a++) {
+            mu[a] = small_u2f(S[a]) / 16.0f;
+            #pragma unroll
+            for (int b = a; b < NC; b++) {
+                const int q = (int)(16u * Q[a][b] - S[a] * S[b]);
+                if (a == b) exact = exact && q < (1 << 20);
+                C[a][b] = small_i2f(q) / 16.0f;
+            }
+        }
+        if (!exact) {
+            #pragma unroll
+            for (int a = 0; a < NC; a++)
+                #pragma unroll
+                for (int b = a; b < NC; b++) C[a][b] = 0.0f;
+            for_texels<UNROLL>([&](int i) {
+                float d[NC];
+                #pragma unroll
+                for (int c = 0; c < NC; c++) d[c] = texel_at_2p15(t[i], c) - (mu[c] + 32768.0f);
+                #pragma unroll
+                for (int a = 0; a < NC; a++)
+                    #pragma unroll
+                    for (int b = a; b < NC; b++) C[a][b] = C[a][b] + d[a] * d[b];
+            });
+        }
     } else {
+        const float cnt = pca_u2f<U2F_BITS>((uint32_t)popc(mask)), cnti = 1.0f / cnt;
         #pragma unroll
         for (int c = 0; c < NC; c++) mu[c] = 0.0f;
         for_texels<UNROLL>([&](int i) {
@@ -57,24 +101,23 @@ ZTC_DEV void pca_endpoints(const Tex &t, uint32_t mask, float lo[4], float hi[4]
                 for (int c = 0; c < NC; c++) mu[c] = mu[c] + div_small(pca_u2f<U2F_BITS>(chan(t[i], c)), cnt, cnti);
             }
         });
-    }
-    // upper triangle only: cov[a][b] and cov[b][a] add bitwise-identical products in the same order
-    float C[NC][NC];
-    #pragma unroll
-    for (int a = 0; a < NC; a++)
+        // upper triangle only: cov[a][b] and cov[b][a] add bitwise-identical products in the same order
         #pragma unroll
-        for (int b = 0; b < NC; b++) C[a][b] = 0.0f;
-    for_texels<UNROLL>([&](int i) {
-        if ((mask >> i) & 1u) {
-            float d[NC];
+        for (int a = 0; a < NC; a++)
             #pragma unroll
-            for (int c = 0; c < NC; c++) d[c] = pca_u2f<U2F_BITS>(chan(t[i], c)) - mu[c];
-            #pragma unroll
-            for (int a = 0; a < NC; a++)
+            for (int b = a; b < NC; b++) C[a][b] = 0.0f;
+        for_texels<UNROLL>([&](int i) {
+            if ((mask >> i) & 1u) {
+                float d[NC];
                 #pragma unroll
-                for (int b = a; b < NC; b++) C[a][b] = C[a][b] + d[a] * d[b];
-        }
-    });
+                for (int c = 0; c < NC; c++) d[c] = pca_u2f<U2F_BITS>(chan(t[i], c)) - mu[c];
+                #pragma unroll
+                for (int a = 0; a < NC; a++)
+                    #pragma unroll
+                    for (int b = a; b < NC; b++) C[a][b] = C[a][b] + d[a] * d[b];
+            }
+        });
+    }
     #pragma unroll
     for (int a = 0; a < NC; a++)
         #pragma unroll
@@ -97,7 +140,10 @@ ZTC_DEV void pca_endpoints(const Tex &t, uint32_t mask, float lo[4], float hi[4]
         if ((mask >> i) & 1u) {
             float s = 0.0f;
             #pragma unroll
-            for (int c = 0; c < NC; c++) s = s + (pca_u2f<U2F_BITS>(chan(t[i], c)) - mu[c]) * ax[c];
+            for (int c = 0; c < NC; c++) {
+                const float d = whole ? texel_at_2p15(t[i], c) - (mu[c] + 32768.0f) : pca_u2f<U2F_BITS>(chan(t[i], c)) - mu[c];
+                s = s + d * ax[c];
+            }
             if (s < tl) tl = s;
             if (s > th) th = s;
         }
