@@ -132,6 +132,12 @@ ZTC_DEV int wunq(int j, int wb) {  // weight n-bit -> 0..64 (power-of-two ranges
     return x > 32 ? x + 1 : x;
 }
 
+// wunq of four weight codes, a byte each, wb = 2..5: the code repeated to 6 bits, plus 1 above 32
+ZTC_DEV uint32_t weight_bytes(uint32_t j, int wb) {
+    const uint32_t x = wb == 2 ? 21u * j : wb == 3 ? 9u * j : wb == 4 ? 4u * j + ((j >> 2) & 0x03030303u) : 2u * j + ((j >> 4) & 0x01010101u);
+    return x + (((x + 0x1F1F1F1Fu) >> 6) & 0x01010101u);
+}
+
 static void build_tables(AstcTables &T) {
     std::memset(&T, 0, sizeof T);
     for (int wb = 2; wb <= 5; wb++)
@@ -192,7 +198,8 @@ __device__ __forceinline__ void load_smem(AstcSmem &S) {
     for (int k = threadIdx.x; k < 256 / 4; k += blockDim.x) ((uint32_t *)S.trit_code)[k] = __ldg((const uint32_t *)gAstc.trit_code + k);
     for (int k = threadIdx.x; k < 128 / 4; k += blockDim.x) ((uint32_t *)S.quint_code)[k] = __ldg((const uint32_t *)gAstc.quint_code + k);
     for (int k = threadIdx.x; k < 128 / 4; k += blockDim.x) ((uint32_t *)&S.wq[0][0])[k] = __ldg((const uint32_t *)&gAstc.wq[0][0] + k);
-    if (threadIdx.x < 8) S.cfg[threadIdx.x] = kAstc.cfg[threadIdx.x];
+    static_assert(sizeof(S.cfg) % 4 == 0 && sizeof(S.cfg) / 4 <= 64, "one word a thread");
+    if (threadIdx.x < sizeof(S.cfg) / 4) ((uint32_t *)S.cfg)[threadIdx.x] = __ldg((const uint32_t *)gAstc.cfg + threadIdx.x);
 }
 
 ZTC_DEV int astc_lerp(int a, int b, int w) { return (((a * 257) * (64 - w) + (b * 257) * w + 32) >> 6) >> 8; }
@@ -229,6 +236,9 @@ ZTC_DEV void endpoint_pair(int cem, const int v[8], int e0[4], int e1[4]) {
     }
 }
 
+// clampi(f2i_x86(y), 0, 255) without a conversion: 0 for NaN and for y from 2^31 on, where f2i_x86 gives INT_MIN
+ZTC_DEV int trunc_to_byte(float y) { return y < 2147483648.0f ? trunc_small(fminf(fmaxf(y, 0.0f), 255.0f)) : 0; }
+
 // float endpoints -> codes + unquantised values of one partition (zap_tex.h:1183-1194)
 ZTC_DEV void astc_quant(const AstcSmem &S, int cfg, int nv, const float lo[4], const float hi[4], int code[8], int uv[8]) {
     float s0 = lo[0] + lo[1] + lo[2], s1 = hi[0] + hi[1] + hi[2];
@@ -237,7 +247,7 @@ ZTC_DEV void astc_quant(const AstcSmem &S, int cfg, int nv, const float lo[4], c
     for (int k = 0; k < 4; k++) {
         if (2 * k >= nv) break;
         float a = keep ? lo[k] : hi[k], b = keep ? hi[k] : lo[k];
-        int x0 = clampi(f2i_x86(a + 0.5f), 0, 255), x1 = clampi(f2i_x86(b + 0.5f), 0, 255);
+        const int x0 = trunc_to_byte(a + 0.5f), x1 = trunc_to_byte(b + 0.5f);
         code[2 * k] = S.q[cfg][x0]; code[2 * k + 1] = S.q[cfg][x1];
         uv[2 * k] = S.uq[cfg][code[2 * k]]; uv[2 * k + 1] = S.uq[cfg][code[2 * k + 1]];
     }
@@ -302,29 +312,31 @@ ZTC_DEV int astc_fit_weights(TexRef ts, uint32_t cm, int cem, int wb, const uint
 // and their 16 best keys instead of a palette and key table of up to 2 x 32 registers.
 template <int LMAX>
 ZTC_DEV int astc_fit_weights_1p(TexRef ts, uint32_t cm, int cem, int wb, const uint8_t *wq, const int uv[8], uint32_t wt[4]) {
+    constexpr int kLog = LMAX == 32 ? 5 : 3;
+    static_assert(LMAX == 1 << kLog, "weight ranges of 8 or 32 levels at most");
     const int L = 1 << wb;
-    int e0[4], e1[4];
-    endpoint_pair(cem, uv, e0, e1);
-    const LerpRow row(e0, e1);
+    int end0[4], end1[4];
+    endpoint_pair(cem, uv, end0, end1);
+    const LerpRow row(end0, end1);
     uint32_t p[16];
-    int best[16];
+    int best[16];  // minus the least key: the key is formed with a shift, and two entries enter by one three-way maximum
     #pragma unroll
-    for (int i = 0; i < 16; i++) { p[i] = ts[i] & cm; best[i] = 0x7FFFFFFF; }
+    for (int i = 0; i < 16; i++) { p[i] = ts[i] & cm; best[i] = (int)0x80000000; }
     #pragma unroll 1
-    for (int j = 0; j < L; j++) {
-        const uint32_t e = row.at(wq[j]) & cm;
-        const int a = (int)dot4(e, e) * LMAX + j;
+    for (int j = 0; j < L; j += 2) {
+        const uint32_t e0 = row.at(wq[j]) & cm, e1 = row.at(wq[j + 1]) & cm;
+        const int a0 = (int)dot4(e0, e0) * LMAX + j, a1 = (int)dot4(e1, e1) * LMAX + j + 1;
         #pragma unroll
-        for (int i = 0; i < 16; i++) best[i] = min(best[i], a - 2 * LMAX * (int)dot4(p[i], e));
+        for (int i = 0; i < 16; i++)
+            best[i] = max3i(best[i], (int)(dot4(p[i], e0) * (2u * LMAX)) - a0, (int)(dot4(p[i], e1) * (2u * LMAX)) - a1);
     }
     int err = 0;
     uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
     #pragma unroll
     for (int i = 0; i < 16; i++) {
-        const int m = best[i];
-        const int q = m >= 0 ? m / LMAX : -((-m + LMAX - 1) / LMAX);
-        err += q + (int)dot4(p[i], p[i]);
-        const uint32_t wi = (uint32_t)(m - q * LMAX);
+        const int m = -best[i];  // (|c|^2 - 2 p.c) LMAX + j
+        err += (m >> kLog) + (int)dot4(p[i], p[i]);
+        const uint32_t wi = (uint32_t)m & (LMAX - 1u);
         if (i < 4) w0 |= wi << (8 * i);
         else if (i < 8) w1 |= wi << (8 * (i - 4));
         else if (i < 12) w2 |= wi << (8 * (i - 8));
@@ -357,21 +369,25 @@ ZTC_DEV bool astc_passes(TexRef ts, const AstcSmem &S, int cfg, int nc, uint32_t
             #pragma unroll
             for (int k = 0; k < PARTS; k++) {
                 const uint32_t m = PARTS == 2 ? (k ? pm : (~pm & 0xFFFFu)) : 0xFFFFu;
-                float aa = 0.0f, ab = 0.0f, bb = 0.0f, sa[4] = {0.0f, 0.0f, 0.0f, 0.0f}, sb[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                uint32_t a0 = wt[0], a1 = wt[1], a2 = wt[2], a3 = wt[3];
-                #pragma unroll 1
-                for (int i = 0; i < 16; i++) {
-                    const uint32_t wi = a0 & 0xFFu;
-                    a0 = (a0 >> 8) | (a1 << 24); a1 = (a1 >> 8) | (a2 << 24); a2 = (a2 >> 8) | (a3 << 24); a3 >>= 8;
-                    if (!((m >> i) & 1u)) continue;
-                    const uint32_t x = ts[i];
-                    float f = (float)wq[wi] / 64.0f, g = 1.0f - f;
-                    aa = aa + g * g; ab = ab + g * f; bb = bb + f * f;
-                    // the alpha sums are computed for CEM 8 too and then not used: each channel's sums are
-                    // independent, so the RGB results are the same as a three-channel loop's
+                // The reference's float sums are exact (weights k / 64, integer texels; see subset_passes in bc7.cu), so
+                // they are integer dot products over the texels of the partition, a byte a texel, scaled.
+                uint32_t W1 = 0u, W2 = 0u, SX[4] = {0u, 0u, 0u, 0u}, SB[4] = {0u, 0u, 0u, 0u};
+                #pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const uint32_t ones = PARTS == 1 ? 0x01010101u : (((m >> (4 * r)) & 15u) * 0x00204081u) & 0x01010101u;
+                    const uint32_t K = weight_bytes(wt[r], wb) & (ones * 255u);
+                    uint32_t x[4];
+                    by_channel(ts[4 * r], ts[4 * r + 1], ts[4 * r + 2], ts[4 * r + 3], x);
+                    W1 = dot4_add(K, 0x01010101u, W1); W2 = dot4_add(K, K, W2);
                     #pragma unroll
-                    for (int c = 0; c < 4; c++) { float xc = (float)chan(x, c); sa[c] = sa[c] + g * xc; sb[c] = sb[c] + f * xc; }
+                    for (int c = 0; c < 4; c++) { SX[c] = dot4_add(x[c], ones, SX[c]); SB[c] = dot4_add(x[c], K, SB[c]); }
                 }
+                const uint32_t n = PARTS == 1 ? 16u : (uint32_t)popc(m);
+                const float aa = small_u2f(4096u * n - 128u * W1 + W2) * (1.0f / 4096.0f), ab = small_u2f(64u * W1 - W2) * (1.0f / 4096.0f);
+                const float bb = small_u2f(W2) * (1.0f / 4096.0f);
+                float sa[4], sb[4];
+                #pragma unroll
+                for (int c = 0; c < 4; c++) { sa[c] = small_u2f(64u * SX[c] - SB[c]) * (1.0f / 64.0f); sb[c] = small_u2f(SB[c]) * (1.0f / 64.0f); }
                 float det = aa * bb - ab * ab;
                 if (det < 1e-6f && det > -1e-6f) continue;
                 float nlo[4], nhi[4];
@@ -556,9 +572,7 @@ __device__ __forceinline__ int astc_single_cta(bool valid, const uint32_t t[16],
         const int e = s_err[k][tid];
         if (e < best) {
             best = e; bc = opaque ? k : 3 + k;
-            int code[1][8];
-            unbytes8(s_code[k][tid], code[0]);
-            astc_codes_bytes<1>(S, bc, code, bcodes);
+            bcodes[0] = (uint32_t)s_code[k][tid]; bcodes[1] = (uint32_t)(s_code[k][tid] >> 32);  // a byte per value, as the block stores them
             const uint4 w = s_wt[k][tid];
             bwt[0] = w.x; bwt[1] = w.y; bwt[2] = w.z; bwt[3] = w.w;
         }
@@ -566,43 +580,89 @@ __device__ __forceinline__ int astc_single_cta(bool valid, const uint32_t t[16],
     return best;
 }
 
-// integer-sequence encoding of n codes (zap_tex.h:1080-1095)
-ZTC_DEV void ise_write(Bits128 &o, const AstcSmem &S, const AstcCfg &c, int n, const uint32_t codes[4]) {
-    const int bits = c.bits, mask = (1 << bits) - 1;
+// The integer sequence of n codes (zap_tex.h:1080-1095) as one 64-bit word: every trial configuration's colour values
+// take at most 64 bits. Value i's low bits start at i * bits plus what the groups before it and the packed code's
+// pieces inside its group take, so only the multiple of `bits` is not known at compile time.
+template <int N>
+ZTC_DEV uint64_t ise_word(const AstcSmem &S, const AstcCfg &c, const uint32_t codes[4]) {
+    const int bits = c.bits;
+    const uint32_t mask = (1u << bits) - 1u;
+    uint64_t acc = 0;
     if (!c.trit && !c.quint) {
-        for (int i = 0; i < n; i++) o.put(get8(codes, i) & (uint32_t)mask, bits);
-        return;
+        #pragma unroll
+        for (int i = 0; i < N; i++) acc |= (uint64_t)get8(codes, i) << (i * bits);
+        return acc;
     }
-    const int gs = c.trit ? 5 : 3, base = c.trit ? 3 : 5;
-    for (int g = 0; g < n; g += gs) {
-        int cnt = min(n - g, gs), key = 0;
-        for (int k = gs - 1; k >= 0; k--) key = key * base + (k < cnt ? (int)(get8(codes, g + k) >> bits) : 0);
-        uint32_t X = c.trit ? S.trit_code[key] : S.quint_code[key];
-        int used = 0;
-        for (int k = 0; k < cnt; k++) {
-            o.put(get8(codes, g + k) & (uint32_t)mask, bits);
-            int xb = c.trit ? (k == 2 || k == 4 ? 1 : 2) : (k == 0 ? 3 : 2);  // packed-code bits after each value
-            o.put((X >> used) & ((1u << xb) - 1u), xb);
-            used += xb;
+    if (c.trit) {  // groups of five: bits, 2, bits, 2, bits, 1, bits, 2, bits, 1
+        #pragma unroll
+        for (int g = 0; g < N; g += 5) {
+            uint32_t key = 0;
+            #pragma unroll
+            for (int k = 4; k >= 0; k--) key = key * 3u + (g + k < N ? get8(codes, g + k) >> bits : 0u);
+            const uint32_t X = S.trit_code[key];
+            #pragma unroll
+            for (int k = 0; k < 5; k++) {
+                if (g + k >= N) break;
+                const int before = k == 0 ? 0 : k == 1 ? 2 : k == 2 ? 4 : k == 3 ? 5 : 7, nx = k == 2 || k == 4 ? 1 : 2;
+                const uint32_t v = (get8(codes, g + k) & mask) | (((X >> before) & ((1u << nx) - 1u)) << bits);
+                acc |= (uint64_t)v << ((g + k) * bits + g / 5 * 8 + before);
+            }
+        }
+    } else {  // groups of three: bits, 3, bits, 2, bits, 2
+        #pragma unroll
+        for (int g = 0; g < N; g += 3) {
+            uint32_t key = 0;
+            #pragma unroll
+            for (int k = 2; k >= 0; k--) key = key * 5u + (g + k < N ? get8(codes, g + k) >> bits : 0u);
+            const uint32_t X = S.quint_code[key];
+            #pragma unroll
+            for (int k = 0; k < 3; k++) {
+                if (g + k >= N) break;
+                const int before = k == 0 ? 0 : k == 1 ? 3 : 5, nx = k == 0 ? 3 : 2;
+                const uint32_t v = (get8(codes, g + k) & mask) | (((X >> before) & ((1u << nx) - 1u)) << bits);
+                acc |= (uint64_t)v << ((g + k) * bits + g / 3 * 7 + before);
+            }
         }
     }
+    return acc;
 }
 
-// block layout (zap_tex.h:1246-1260): mode, partitions, seed / CEM, ISE colours, weights reversed from bit 127
+// block layout (zap_tex.h:1246-1260): mode, partitions, seed / CEM, the colour values' integer sequence, and the weights
+// as bits running down from bit 127. N: colour values at most (bytes of codes past the configuration's are zero).
+template <int PARTS>
 ZTC_DEV uint4 astc_pack(const AstcSmem &S, int cfg, int seed, const uint32_t codes[4], const uint32_t wt[4]) {
     const AstcCfg c = S.cfg[cfg];
-    const int R = c.wb == 2 ? 4 : c.wb == 3 ? 7 : c.wb == 4 ? 4 : 7, H = c.wb >= 4 ? 1 : 0;
-    uint32_t mode = (uint32_t)(((R >> 1) & 1) | (((R >> 2) & 1) << 1) | ((R & 1) << 4) | (2 << 5) | (H << 9));
-    Bits128 o;
-    o.put(mode, 11);
-    o.put((uint32_t)(c.parts - 1), 2);
-    if (c.parts == 2) { o.put((uint32_t)seed, 10); o.put((uint32_t)c.cem << 2, 6); }
-    else o.put((uint32_t)c.cem, 4);
-    ise_write(o, S, c, c.nv * c.parts, codes);
-    Bits128 ws;
-    for (int i = 0; i < 16; i++) ws.put(get8(wt, i), c.wb);
-    // stream bit i -> block bit 127 - i
-    return make_uint4(o.w[0] | brev(ws.w[3]), o.w[1] | brev(ws.w[2]), o.w[2] | brev(ws.w[1]), o.w[3] | brev(ws.w[0]));
+    const int wb = c.wb, R = wb == 2 ? 4 : wb == 3 ? 7 : wb == 4 ? 4 : 7, H = wb >= 4 ? 1 : 0;
+    const uint32_t mode = (uint32_t)(((R >> 1) & 1) | (((R >> 2) & 1) << 1) | ((R & 1) << 4) | (2 << 5) | (H << 9));
+    uint64_t lo, hi = 0, ise;
+    int pos;
+    if (PARTS == 2) {
+        lo = mode | (1u << 11) | ((uint32_t)seed << 13) | ((uint64_t)((uint32_t)c.cem << 2) << 23);
+        pos = 29;
+        ise = ise_word<12>(S, c, codes);
+    } else {
+        lo = mode | ((uint32_t)c.cem << 13);
+        pos = 17;
+        ise = c.nv == 6 ? ise_word<6>(S, c, codes) : ise_word<8>(S, c, codes);
+    }
+    lo |= ise << pos;
+    hi |= ise >> (64 - pos);
+    uint64_t w = 0, top = 0;  // the weights' bits from the least: texel i at i * wb (w), and past 64 bits (top)
+    #pragma unroll
+    for (int r = 0; r < 4; r++) {  // a row's four codes, a byte each, drawn together to 4 wb bits
+        const uint32_t t = (wt[r] & 0x00FF00FFu) | (((wt[r] >> 8) & 0x00FF00FFu) << wb);
+        const uint64_t row = (t & 0xFFFFu) | ((t >> 16) << (2 * wb));
+        w |= row << (4 * wb * r);
+        if (r == 3 && wb == 5) top = row >> 4;
+    }
+    const uint32_t h0 = brev((uint32_t)(w >> 32)), h1 = brev((uint32_t)w);  // stream bit i -> block bit 127 - i
+    hi |= (uint64_t)h0 | ((uint64_t)h1 << 32);
+    lo |= (uint64_t)brev((uint32_t)top) << 32;
+    return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+}
+// one partition (the form the host test of the block logic calls)
+ZTC_DEV uint4 astc_pack(const AstcSmem &S, int cfg, int seed, const uint32_t codes[4], const uint32_t wt[4]) {
+    return astc_pack<1>(S, cfg, seed, codes, wt);
 }
 
 __global__ void __launch_bounds__(128, ZTC_MINB_ASTC_SINGLE) astc_single_kernel(SrcU8 src, int bw, int by0, int nblocks, uint8_t *__restrict__ out,
@@ -768,7 +828,7 @@ __global__ void __launch_bounds__(128) astc_two_part_kernel(SrcU8 src, int bw, i
         uint32_t key = (pj >= 0 && e < best) ? (((uint32_t)e << 3) | (uint32_t)l) : 0xFFFFFFFFu;
         #pragma unroll
         for (int m = 1; m < kAstcGroup; m <<= 1) key = min(key, __shfl_xor_sync(gmask, key, m, kAstcGroup));
-        if (key != 0xFFFFFFFFu && (int)(key & 7u) == l) store_block16(out + (size_t)b * 16, astc_pack(S, cfg, pseed[pj], codes, wt));
+        if (key != 0xFFFFFFFFu && (int)(key & 7u) == l) store_block16(out + (size_t)b * 16, astc_pack<2>(S, cfg, pseed[pj], codes, wt));
     }
 }
 
