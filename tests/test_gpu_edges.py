@@ -82,3 +82,20 @@ def test_scratch_pool_across_streams_threads_and_capture(cuda_lib, oracle):
         g.replay()
         torch.cuda.synchronize()
         assert np.array_equal(out.cpu().numpy(), want[0])
+
+
+@pytest.mark.parametrize("fmt", [zap_b200.BC1, zap_b200.BC3])
+@pytest.mark.parametrize("size", [(1, 1), (4, 4), (13, 6), (64, 20), (252, 260), (640, 592), (640, 596), (1200, 1060)])
+def test_colour_blocks_around_the_launch_rule(cuda_lib, oracle, fmt, size):
+    """Eight threads per block up to 23680 blocks (160 per SM of 148), one above: both sides of the line, partial CTAs, noise
+    (wide channels, long climbs), flat and two-colour blocks."""
+    w, h = size
+    rng = np.random.default_rng(w * 7 + h + fmt)
+    img = _image(w, h, w + h)
+    bw, bh = (w + 3) // 4, (h + 3) // 4
+    kind = np.kron(rng.integers(0, 4, (bh, bw)), np.ones((4, 4), int))[:h, :w]
+    flat = np.kron(rng.integers(0, 256, (bh, bw, 4)), np.ones((4, 4, 1), int))[:h, :w].astype(np.uint8)
+    near = (flat.astype(int) + rng.integers(-6, 7, (h, w, 4))).clip(0, 255).astype(np.uint8)
+    img = np.where((kind == 1)[..., None], flat, np.where((kind == 2)[..., None], near, img))
+    img = np.where(((kind == 3) & (rng.random((h, w)) < 0.5))[..., None], flat, img)
+    assert np.array_equal(zap_b200.bc_encode_dev(torch.from_numpy(img).cuda(), fmt).cpu().numpy(), oracle.bc_encode(img, fmt))

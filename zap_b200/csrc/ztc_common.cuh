@@ -287,6 +287,14 @@ ZTC_DEV float texel_at_2p15(uint32_t x, int c) {
     return u_as_f(0x47000000u | (((x >> (8 * c)) & 0xFFu) << 8));
 #endif
 }
+// channel c of texel x as a float
+ZTC_DEV float byte_u2f(uint32_t x, int c) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7440u | (uint32_t)c)) - 8388608.0f;
+#else
+    return (float)((x >> (8 * c)) & 0xFFu);
+#endif
+}
 // an integer in (-2^22, 2^22) as a float
 ZTC_DEV float small_i2f(int n) { return u_as_f(0x4B400000u + (uint32_t)n) - 12582912.0f; }
 
