@@ -99,3 +99,34 @@ def test_colour_blocks_around_the_launch_rule(cuda_lib, oracle, fmt, size):
     img = np.where((kind == 1)[..., None], flat, np.where((kind == 2)[..., None], near, img))
     img = np.where(((kind == 3) & (rng.random((h, w)) < 0.5))[..., None], flat, img)
     assert np.array_equal(zap_b200.bc_encode_dev(torch.from_numpy(img).cuda(), fmt).cpu().numpy(), oracle.bc_encode(img, fmt))
+
+
+def _hard_opaque(w, h, seed, share):
+    """An opaque image of which about `share` of the blocks are noise or two far colours (the second searches of ASTC and BC7),
+    the rest smooth."""
+    rng = np.random.default_rng(seed)
+    bw, bh = (w + 3) // 4, (h + 3) // 4
+    y, x = np.mgrid[0:h, 0:w]
+    img = np.stack([x * 255 // max(w, 2), y * 255 // max(h, 2), (x + y) % 256, np.full((h, w), 255)], 2).astype(np.uint8)
+    pick = np.kron(rng.random((bh, bw)) < share, np.ones((4, 4), bool))[:h, :w]
+    two = np.kron(rng.random((bh, bw)) < 0.5, np.ones((4, 4), bool))[:h, :w]
+    a, b = (np.kron(rng.integers(0, 256, (bh, bw, 3)), np.ones((4, 4, 1), int))[:h, :w] for _ in range(2))
+    mix = np.where((rng.random((h, w)) < 0.5)[..., None], a, b)
+    noise = rng.integers(0, 256, (h, w, 3))
+    img[..., :3] = np.where(pick[..., None], np.where(two[..., None], mix, noise), img[..., :3])
+    return img
+
+
+@pytest.mark.parametrize("size,share", [((4, 4), 1.0), ((21, 13), 1.0), ((64, 64), 0.3), ((136, 136), 1.0), ((140, 140), 1.0),
+                                        ((1024, 512), 0.01), ((1024, 512), 0.2)])
+@pytest.mark.parametrize("opaque", [True, False])
+def test_second_search_around_the_list_rule(cuda_lib, oracle, size, share, opaque):
+    """ASTC's two-partition search and BC7's modes 5 and 1, a CTA per listed block while the list has no more blocks than the
+    launch CTAs (1184), a group of lanes per block above: lists of one block, on either side of the line, and long ones."""
+    w, h = size
+    img = _hard_opaque(w, h, w + h, share)
+    if not opaque:
+        img[..., 3] = np.random.default_rng(3).integers(200, 256, (h, w))
+    t = torch.from_numpy(img).cuda()
+    assert np.array_equal(zap_b200.astc_encode_dev(t).cpu().numpy(), oracle.astc_encode(img))
+    assert np.array_equal(zap_b200.bc_encode_dev(t, zap_b200.BC7).cpu().numpy(), oracle.bc_encode(img, zap_b200.BC7))
