@@ -130,3 +130,19 @@ def test_second_search_around_the_list_rule(cuda_lib, oracle, size, share, opaqu
     t = torch.from_numpy(img).cuda()
     assert np.array_equal(zap_b200.astc_encode_dev(t).cpu().numpy(), oracle.astc_encode(img))
     assert np.array_equal(zap_b200.bc_encode_dev(t, zap_b200.BC7).cpu().numpy(), oracle.bc_encode(img, zap_b200.BC7))
+
+
+@pytest.mark.parametrize("size", [(1, 1), (9, 5), (61, 33), (532, 532), (536, 536), (1500, 1212), (1504, 1212)])
+def test_bc7_around_the_launch_rules(cuda_lib, oracle, size):
+    """Mode 6 by eight threads per block up to 17760 blocks (120 per SM of 148), in small CTAs up to 113664, in large ones
+    above; channels wide enough that their sums are taken in float order, flat blocks and smooth ones in one image."""
+    w, h = size
+    rng = np.random.default_rng(w + h)
+    bw, bh = (w + 3) // 4, (h + 3) // 4
+    kind = np.kron(rng.integers(0, 8, (bh, bw)), np.ones((4, 4), int))[:h, :w, None]
+    flat = np.kron(rng.integers(0, 256, (bh, bw, 4)), np.ones((4, 4, 1), int))[:h, :w]
+    near = flat + rng.integers(-9, 10, (h, w, 4))
+    wide = np.where(rng.random((h, w, 4)) < 0.5, flat, 255 - flat)
+    img = np.where(kind == 0, wide, np.where(kind == 1, flat, near)).clip(0, 255).astype(np.uint8)
+    img[..., 3] = np.where(kind[..., 0] % 3 == 0, 255, img[..., 3])
+    assert np.array_equal(zap_b200.bc_encode_dev(torch.from_numpy(img).cuda(), zap_b200.BC7).cpu().numpy(), oracle.bc_encode(img, zap_b200.BC7))

@@ -8,7 +8,7 @@
 //                on the other, combined per rotation;
 //        mode 1  the opaque ones, an 8-lane group per block: the 64 partitions are scored 8 per lane, the top 4 by
 //                (score, partition) are merged across the group, then lane = (candidate, subset) fits the 8
-//                subsets; with at most one listed block per CTA, the CTA's 64 threads score one partition each.
+//                subsets; a list of at most one block per CTA gives each block a whole CTA (hard_block).
 //      Decoded SSE checks of the reference (zap__bc7_err, zap_tex.h:761,780) equal the fit SSE here: the expand and
 //      interpolation are the decoder's, anchor swaps preserve decoded values because every weight table satisfies
 //      w(n-1-j) = 64 - w(j), mode 1 shares its p-bit between a subset's endpoints, and mode 1 decodes alpha 255
@@ -313,10 +313,175 @@ __global__ void __launch_bounds__(CTA, mode6_min_ctas<CTA>()) bc7_mode6_kernel(S
     }
 }
 
+// ---------------------------------------------------------------- mode 6 in small launches: eight threads per block
+// With fewer blocks than the chip has room for threads, a launch takes as long as one thread's chain of dependent work. Here
+// thread j of a block's eight has channel j & 3 and endpoint j >> 2 for the solves and quantisation, two entries of
+// the palette to build, and two texels (row j & 3, columns 2 (j >> 2) and on) to fit; sums, minima and packed words go over
+// the eight by shuffles. Every float is the one-thread code's (the sums over threads are of integers). All loops run
+// until no block of the warp needs them.
+constexpr unsigned kAllLanes = 0xFFFFFFFFu;
+template <typename T>
+__device__ __forceinline__ T add8(T v) {
+    #pragma unroll
+    for (int m = 1; m < 8; m <<= 1) v += __shfl_xor_sync(kAllLanes, v, m);
+    return v;
+}
+__device__ __forceinline__ uint32_t or8(uint32_t v) {
+    #pragma unroll
+    for (int m = 1; m < 8; m <<= 1) v |= __shfl_xor_sync(kAllLanes, v, m);
+    return v;
+}
+struct Mode6Group {           // a block's shared words
+    uint32_t px[16];          // its texels
+    uint4 ch[4];              // and by channel, a byte per texel
+    uint4 pal[4]; int4 A[4];  // the palette, and 16 |entry|^2 + index
+};
+// returns the SSE; blk: the block (the same in all eight threads)
+__device__ __forceinline__ int mode6_encode_group(Mode6Group &G, uint4 &blk) {
+    const int j = threadIdx.x & 7, c = j & 3, end = j >> 2, base = threadIdx.x & 31 & ~7;
+    float mu[4], ax[4];
+    pca_axis<4, 1>(TexRef{G.px, 1}, mu, ax);
+    float n2 = 0.0f, tl = 1e9f, th = -1e9f;
+    #pragma unroll
+    for (int k = 0; k < 4; k++) n2 = n2 + ax[k] * ax[k];
+    const int i0 = 4 * c + 2 * end;  // this thread's texels i0, i0 + 1
+    const uint32_t p[2] = {G.px[i0], G.px[i0 + 1]};
+    #pragma unroll
+    for (int i = 0; i < 2; i++) {
+        float s = 0.0f;
+        #pragma unroll
+        for (int k = 0; k < 4; k++) s = s + (texel_at_2p15(p[i], k) - (mu[k] + 32768.0f)) * ax[k];
+        if (s < tl) tl = s;
+        if (s > th) th = s;
+    }
+    #pragma unroll
+    for (int m = 1; m < 8; m <<= 1) {
+        tl = fminf(tl, __shfl_xor_sync(kAllLanes, tl, m));
+        th = fmaxf(th, __shfl_xor_sync(kAllLanes, th, m));
+    }
+    const float muc = c == 0 ? mu[0] : c == 1 ? mu[1] : c == 2 ? mu[2] : mu[3], axc = c == 0 ? ax[0] : c == 1 ? ax[1] : c == 2 ? ax[2] : ax[3];
+    float v = muc + axc * (end ? th : tl) / n2;  // this thread's endpoint channel
+    const uint4 chan4 = G.ch[c];
+    const uint32_t x4[4] = {chan4.x, chan4.y, chan4.z, chan4.w};
+    const uint32_t SX = dot4_add(x4[3], 0x01010101u, dot4_add(x4[2], 0x01010101u, dot4_add(x4[1], 0x01010101u, dot4(x4[0], 0x01010101u))));
+    const int pp = (int)(dot4(p[0], p[0]) + dot4(p[1], p[1]));
+    int err = 0;
+    uint32_t lo8 = 0, hi8 = 0, ilo = 0, ihi = 0;  // the accepted endpoints (8 bits a channel) and indices
+    bool go = true;
+    #pragma unroll 1
+    for (int it = 0; it < 3; it++) {
+        if (it > 0) {  // least-squares refit (subset_passes)
+            go = go && err > 0;
+            if (!__any_sync(kAllLanes, go)) break;
+            uint32_t W1 = 0u, W2 = 0u, SB = 0u;
+            #pragma unroll
+            for (int r = 0; r < 4; r++) {
+                uint32_t k = ((r < 2 ? ilo : ihi) >> (16 * (r & 1))) & 0xFFFFu;
+                k = (k | (k << 8)) & 0x00FF00FFu;
+                k = (k | (k << 4)) & 0x0F0F0F0Fu;
+                const uint32_t K = 4u * k + (((k + 0x02020202u) >> 2) & 0x07070707u);
+                W1 = dot4_add(K, 0x01010101u, W1); W2 = dot4_add(K, K, W2); SB = dot4_add(x4[r], K, SB);
+            }
+            const float aa = small_u2f(65536u - 128u * W1 + W2) * (1.0f / 4096.0f), ab = small_u2f(64u * W1 - W2) * (1.0f / 4096.0f);
+            const float bb = small_u2f(W2) * (1.0f / 4096.0f), det = aa * bb - ab * ab;
+            go = go && !(det < 1e-6f && det > -1e-6f);
+            const float sa = small_u2f(64u * SX - SB) * (1.0f / 64.0f), sb = small_u2f(SB) * (1.0f / 64.0f);
+            const float nv = clamp255((end ? sb * aa - sa * ab : sa * bb - sb * ab) / det);
+            v = go ? nv : 0.0f;  // 0 where the result is not used (a singular system's could be NaN)
+        }
+        const float v4[4] = {v, 0.0f, 0.0f, 0.0f};
+        uint32_t k2[2][4];
+        int e2[2];
+        quant8_pbits<1>(v4, k2, e2);
+        #pragma unroll
+        for (int m = 1; m < 4; m <<= 1) {  // over the endpoint's four channels
+            e2[0] += __shfl_xor_sync(kAllLanes, e2[0], m);
+            e2[1] += __shfl_xor_sync(kAllLanes, e2[1], m);
+        }
+        const uint32_t pb = e2[1] < e2[0] ? 1u : 0u;
+        const uint32_t mine = (2u * ((pb ? k2[1][0] : k2[0][0]) & 127u) + pb) << (8 * c);
+        const uint32_t nlo = or8(end ? 0u : mine), nhi = or8(end ? mine : 0u);
+        if (it > 0) {
+            go = go && !(nlo == lo8 && nhi == hi8);  // the accepted endpoints again: the refits end
+            if (!__any_sync(kAllLanes, go)) break;
+        }
+        const int x0[4] = {(int)chan(nlo, 0), (int)chan(nlo, 1), (int)chan(nlo, 2), (int)chan(nlo, 3)};
+        const int x1[4] = {(int)chan(nhi, 0), (int)chan(nhi, 1), (int)chan(nhi, 2), (int)chan(nhi, 3)};
+        const Lerp4 row(x0, x1);
+        __syncwarp();  // the last pass's reads of the palette are done
+        #pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint32_t e = row.at(w4(2 * j + k));
+            ((uint32_t *)G.pal)[2 * j + k] = e;
+            ((int *)G.A)[2 * j + k] = (int)dot4(e, e) * 16 + 2 * j + k;
+        }
+        __syncwarp();
+        int m0 = (int)0x80000000, m1 = (int)0x80000000;  // minus the least keys (palette_fit)
+        #pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint4 e = G.pal[k];
+            const int4 a = G.A[k];
+            m0 = max3i(m0, (int)(dot4(p[0], e.x) << 5) - a.x, (int)(dot4(p[0], e.y) << 5) - a.y);
+            m1 = max3i(m1, (int)(dot4(p[1], e.x) << 5) - a.x, (int)(dot4(p[1], e.y) << 5) - a.y);
+            m0 = max3i(m0, (int)(dot4(p[0], e.z) << 5) - a.z, (int)(dot4(p[0], e.w) << 5) - a.w);
+            m1 = max3i(m1, (int)(dot4(p[1], e.z) << 5) - a.z, (int)(dot4(p[1], e.w) << 5) - a.w);
+        }
+        const int ne = add8((-m0 >> 4) + (-m1 >> 4) + pp);
+        const uint32_t two = ((uint32_t)-m0 & 15u) | (((uint32_t)-m1 & 15u) << 4);
+        const uint32_t nilo = or8(i0 < 8 ? two << (4 * i0) : 0u), nihi = or8(i0 < 8 ? 0u : two << (4 * (i0 - 8)));
+        go = go && (it == 0 || ne < err);
+        if (go) { err = ne; lo8 = nlo; hi8 = nhi; ilo = nilo; ihi = nihi; }
+    }
+    int q[2][4], pb[2] = {(int)(lo8 & 1u), (int)(hi8 & 1u)};
+    #pragma unroll
+    for (int k = 0; k < 4; k++) { q[0][k] = (int)chan(lo8, k) >> 1; q[1][k] = (int)chan(hi8, k) >> 1; }
+    blk = pack_mode6_block(q, pb, (uint64_t)ilo | ((uint64_t)ihi << 32));
+    (void)base;
+    return err;
+}
+
+constexpr int kGroupBlocks6 = 16;  // blocks of a 128-thread CTA
+__global__ void __launch_bounds__(8 * kGroupBlocks6) bc7_mode6_group_kernel(SrcU8 src, int bw, int by0, int nblocks, BlockOut out, size_t b0,
+                                                                            uint32_t *__restrict__ count, uint2 *__restrict__ items) {
+    __shared__ Mode6Group G[kGroupBlocks6];
+    const int slot = threadIdx.x >> 3, j = threadIdx.x & 7, lane = threadIdx.x & 31, bi = blockIdx.x * kGroupBlocks6 + slot;
+    const int b = min(bi, nblocks - 1);  // threads past the last block repeat it and store nothing
+    Mode6Group &M = G[slot];
+    if (j < 4) {
+        uint32_t t[4], x[4];
+        gather_row(src, b % bw, by0 + b / bw, j, t);
+        by_channel(t[0], t[1], t[2], t[3], x);
+        #pragma unroll
+        for (int i = 0; i < 4; i++) { M.px[4 * j + i] = t[i]; ((uint32_t *)&M.ch[i])[j] = x[i]; }
+    }
+    __syncwarp();
+    uint4 blk;
+    const int err = mode6_encode_group(M, blk);
+    const bool store = j == 0 && bi < nblocks, hard = store && err > 16 * 4;  // zap_tex.h:758 early exit
+    if (store) put_block16(out, b0 + (size_t)b, blk);
+    const unsigned ballot = __ballot_sync(kAllLanes, hard);
+    if (ballot) {
+        const int leader = __ffs(ballot) - 1;
+        uint32_t first = 0;
+        if (lane == leader) first = atomicAdd(count, (uint32_t)__popc(ballot));
+        first = __shfl_sync(kAllLanes, first, leader);
+        const int pos = (int)first + __popc(ballot & ((1u << lane) - 1u));
+        if (hard && ZTC_IN_BOUNDS(pos, nblocks, 6)) items[pos] = make_uint2((uint32_t)b, (uint32_t)err);
+    }
+}
+
+// Blocks per SM up to which mode 6 takes eight threads per block. Whole encodes, one / eight threads per block: 64x64 31.2 / 25.4
+// us, 256x256 33.7 / 27.9, 512x512 36.5 / 35.5, 724x724 36.3 / 42.3, 1024x1024 42.3 / 58.7.
+constexpr int kGroupLimit6 = 120;
+// Blocks per SM above which the large CTAs are taken: one wave of small ones is 768. Between that and a wave of
+// large ones (896) the small ones would run a second, nearly empty wave (1918x1077 74.3 -> 68.9 us, 1440x1440 57.9 -> 53.0).
+constexpr int kLargeFrom6 = 768;
 // the mode-6 launch, at the CTA size that suits its block count
 cudaError_t launch_mode6(const SrcU8 &src, int bw, int by0, int nblocks, const BlockOut &out, size_t b0, uint32_t *count, uint2 *items,
                          cudaStream_t s) {
-    if (nblocks >= ztc_sm_count() * mode6_min_ctas<kMode6Large>() * kMode6Large)
+    if (nblocks <= ztc_sm_count() * kGroupLimit6)
+        bc7_mode6_group_kernel<<<(nblocks + kGroupBlocks6 - 1) / kGroupBlocks6, 8 * kGroupBlocks6, 0, s>>>(src, bw, by0, nblocks, out, b0, count, items);
+    else if (nblocks > ztc_sm_count() * kLargeFrom6)
         bc7_mode6_kernel<kMode6Large><<<(nblocks + kMode6Large - 1) / kMode6Large, kMode6Large, 0, s>>>(src, bw, by0, nblocks, out, b0, count, items);
     else
         bc7_mode6_kernel<kMode6Small><<<(nblocks + kMode6Small - 1) / kMode6Small, kMode6Small, 0, s>>>(src, bw, by0, nblocks, out, b0, count, items);
@@ -341,25 +506,39 @@ ZTC_DEV uint32_t rotate_texel(uint32_t v, int rot) {  // mode 5 rotation: swap A
 // (rotated A, 8-bit endpoints): the alpha part's loops run over its one channel.
 constexpr int kPartColour = 1, kPartAlpha = 2;
 
+// one endpoint value: finite v within [-510, 765] (clamped least-squares endpoints, or the starts), as for quant_pbit
+ZTC_DEV void m5_quant1(float v, int n, int &q, int &x8) {
+    const int top = (1 << n) - 1;
+    const float gv = div255(v * (float)top) + 0.5f;
+    ZTC_TRUNC_DOMAIN(gv);
+    int g = trunc_mid(gv), bq = 0, bd = 1 << 30;
+    #pragma unroll
+    for (int k = 0; k < 3; k++) {
+        int tq = clampi(around(g, k), 0, top);
+        const float dv = fabsf(small_u2f((uint32_t)expand_bits(tq, n)) - v);
+        ZTC_TRUNC_DOMAIN(dv);
+        int d = trunc_small(dv);
+        if (d < bd) { bd = d; bq = tq; }
+    }
+    q = bq; x8 = expand_bits(bq, n);
+}
 template <int KIND>
 ZTC_DEV void m5_quant(const float v[3], int nc, int n, int q[3], int x8[3]) {
-    const int top = (1 << n) - 1;
     #pragma unroll
     for (int c = 0; c < 3; c++) {
         if (c >= nc || (KIND == kPartAlpha && c > 0)) { q[c] = 0; x8[c] = 0; continue; }
-        // finite v within [-510, 765] (clamped least-squares endpoints, or the starts), as for quant_pbit
-        const float gv = div255(v[c] * (float)top) + 0.5f;
-        ZTC_TRUNC_DOMAIN(gv);
-        int g = trunc_mid(gv), bq = 0, bd = 1 << 30;
+        m5_quant1(v[c], n, q[c], x8[c]);
+    }
+}
+// the part's four entries and 4 |entry|^2 + index
+template <int KIND>
+ZTC_DEV void m5_palette(const int x0[3], const int x1[3], uint32_t pal[4], int A[4]) {
+    #pragma unroll
+    for (int j = 0; j < 4; j++) {
+        uint32_t e = 0;
         #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            int tq = clampi(around(g, k), 0, top);
-            const float dv = fabsf(small_u2f((uint32_t)expand_bits(tq, n)) - v[c]);
-            ZTC_TRUNC_DOMAIN(dv);
-            int d = trunc_small(dv);
-            if (d < bd) { bd = d; bq = tq; }
-        }
-        q[c] = bq; x8[c] = expand_bits(bq, n);
+        for (int c = 0; c < (KIND == kPartAlpha ? 1 : 3); c++) e |= (uint32_t)lerp64(x0[c], x1[c], w2(j)) << (8 * c);
+        pal[j] = e; A[j] = (int)dot4(e, e) * 4 + j;
     }
 }
 // The part's texels p[16] are in registers (the colour part: rotated RGB in the low three bytes; the alpha part:
@@ -369,13 +548,7 @@ template <int KIND>
 ZTC_DEV int m5_fit(const uint32_t p[16], const int x0[3], const int x1[3], uint32_t &idx) {
     uint32_t pal[4];
     int A[4];
-    #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        uint32_t e = 0;
-        #pragma unroll
-        for (int c = 0; c < (KIND == kPartAlpha ? 1 : 3); c++) e |= (uint32_t)lerp64(x0[c], x1[c], w2(j)) << (8 * c);
-        pal[j] = e; A[j] = (int)dot4(e, e) * 4 + j;
-    }
+    m5_palette<KIND>(x0, x1, pal, A);
     int err = 0;
     uint32_t bits = 0;
     #pragma unroll
@@ -389,30 +562,31 @@ ZTC_DEV int m5_fit(const uint32_t p[16], const int x0[3], const int x1[3], uint3
     return err;
 }
 // Least-squares endpoints for fixed 2-bit indices (zap_tex.h:636-648). The reference sums floats, but every one of
-// its sums is exact: w = k / 64 with k in {0, 21, 43, 64} and u = 1 - w, so u*u, u*w and w*w are multiples of 2^-12
-// below 1, u*x and w*x multiples of 2^-6 below 256, and no partial sum of 16 terms needs more than 24 bits in those
-// units. Integer sums scaled by 2^-12 and 2^-6 are therefore the reference's floats, bit for bit, in any order.
+// its sums is exact (see subset_passes), so they are integer dot products, a byte a texel, scaled. x[c]: the part's
+// channel c, row by row; sx[c]: its sum.
 template <int KIND>
-ZTC_DEV bool m5_lsq(const uint32_t p[16], int nc, uint32_t idx, float lo[3], float hi[3]) {
+ZTC_DEV bool m5_lsq(const uint32_t x[3][4], const uint32_t sx[3], uint32_t idx, float lo[3], float hi[3]) {
     constexpr int kC = KIND == kPartAlpha ? 1 : 3;
-    int aa = 0, ab = 0, bb = 0, sa[3] = {0, 0, 0}, sb[3] = {0, 0, 0};
+    uint32_t W1 = 0u, W2 = 0u, SB[3] = {0u, 0u, 0u};
     #pragma unroll
-    for (int i = 0; i < 16; i++) {
-        const int k = (int)((0x402B1500u >> (8 * ((idx >> (2 * i)) & 3u))) & 0xFFu), u = 64 - k;  // w2: 0, 21, 43, 64
-        aa += u * u; ab += u * k; bb += k * k;
+    for (int r = 0; r < 4; r++) {
+        uint32_t j = (idx >> (8 * r)) & 0xFFu;
+        j = (j | (j << 12)) & 0x000F000Fu;
+        j = (j | (j << 6)) & 0x03030303u;
+        const uint32_t K = 21u * j + ((j >> 1) & 0x01010101u);  // w2: 0, 21, 43, 64
+        W1 = dot4_add(K, 0x01010101u, W1); W2 = dot4_add(K, K, W2);
         #pragma unroll
-        for (int c = 0; c < kC; c++) { const int x = (int)chan(p[i], c); sa[c] += u * x; sb[c] += k * x; }
+        for (int c = 0; c < kC; c++) SB[c] = dot4_add(x[c][r], K, SB[c]);
     }
-    const float faa = small_u2f((uint32_t)aa) * (1.0f / 4096.0f), fab = small_u2f((uint32_t)ab) * (1.0f / 4096.0f),
-                fbb = small_u2f((uint32_t)bb) * (1.0f / 4096.0f);  // sums below 2^17
+    const float faa = small_u2f(65536u - 128u * W1 + W2) * (1.0f / 4096.0f), fab = small_u2f(64u * W1 - W2) * (1.0f / 4096.0f),
+                fbb = small_u2f(W2) * (1.0f / 4096.0f);  // sums below 2^17
     float det = faa * fbb - fab * fab;
     if (det < 1e-6f && det > -1e-6f) return false;
     #pragma unroll
-    for (int c = 0; c < kC; c++)
-        if (c < nc) {
-            const float fa = small_u2f((uint32_t)sa[c]) * (1.0f / 64.0f), fb = small_u2f((uint32_t)sb[c]) * (1.0f / 64.0f);  // below 2^18
-            lo[c] = clamp255((fa * fbb - fb * fab) / det); hi[c] = clamp255((fb * faa - fa * fab) / det);
-        }
+    for (int c = 0; c < kC; c++) {
+        const float fa = small_u2f(64u * sx[c] - SB[c]) * (1.0f / 64.0f), fb = small_u2f(SB[c]) * (1.0f / 64.0f);  // below 2^18
+        lo[c] = clamp255((fa * fbb - fb * fab) / det); hi[c] = clamp255((fb * faa - fa * fab) / det);
+    }
     return true;
 }
 // quantise, fit, up to two least-squares refits (zap_tex.h:626-657); lo / hi: the start endpoints
@@ -421,9 +595,17 @@ ZTC_DEV int m5_part(const uint32_t p[16], float lo[3], float hi[3], int q[2][3],
     constexpr bool alpha = KIND == kPartAlpha;
     const int nc = alpha ? 1 : 3, n = alpha ? 8 : 7;
     int err = 0;
+    uint32_t x[3][4], sx[3] = {0u, 0u, 0u};  // the texels by channel (m5_lsq)
+    #pragma unroll
+    for (int r = 0; r < 4; r++) {
+        uint32_t w[4];
+        by_channel(p[4 * r], p[4 * r + 1], p[4 * r + 2], p[4 * r + 3], w);
+        #pragma unroll
+        for (int c = 0; c < (alpha ? 1 : 3); c++) { x[c][r] = w[c]; sx[c] = dot4_add(w[c], 0x01010101u, sx[c]); }
+    }
     #pragma unroll 1
     for (int it = 0; it < 3; it++) {
-        if (it > 0 && !m5_lsq<KIND>(p, nc, idx, lo, hi)) break;
+        if (it > 0 && !m5_lsq<KIND>(x, sx, idx, lo, hi)) break;
         int tq[2][3], x0[3], x1[3];
         m5_quant<KIND>(lo, nc, n, tq[0], x0); m5_quant<KIND>(hi, nc, n, tq[1], x1);
         if (it > 0) {  // the accepted endpoints again: the same fit and SSE, which ends the refits
@@ -491,65 +673,60 @@ constexpr int kMode1Tries = 4;  // partitions fully fitted after ranking (ZAP__B
 
 __device__ __forceinline__ bool mode1_fits(TexRef ts, const int cand[kMode1Tries], int &err, uint4 &blk, const int l, const unsigned gmask);
 
+// The reference's nine float moment sums over the texels in `mask` (r, g, b, rr, gg, bb, rg, rb, gb): integers below 2^24,
+// so exact in any order: dot products over the texels by channel (x[c], a byte a texel), the texels outside masked
+// out (about 60 operations instead of 560).
+__device__ __forceinline__ void subset_moments(const uint4 x[3], uint32_t mask, float s[9]) {
+    uint32_t S[3] = {0u, 0u, 0u}, Q[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+    const uint32_t w[3][4] = {{x[0].x, x[0].y, x[0].z, x[0].w}, {x[1].x, x[1].y, x[1].z, x[1].w}, {x[2].x, x[2].y, x[2].z, x[2].w}};
+    #pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const uint32_t m = ((((mask >> (4 * r)) & 15u) * 0x00204081u) & 0x01010101u) * 255u;
+        const uint32_t R = w[0][r] & m, G = w[1][r] & m, B = w[2][r] & m;
+        S[0] = dot4_add(R, 0x01010101u, S[0]); S[1] = dot4_add(G, 0x01010101u, S[1]); S[2] = dot4_add(B, 0x01010101u, S[2]);
+        Q[0] = dot4_add(R, R, Q[0]); Q[1] = dot4_add(G, G, Q[1]); Q[2] = dot4_add(B, B, Q[2]);
+        Q[3] = dot4_add(R, G, Q[3]); Q[4] = dot4_add(R, B, Q[4]); Q[5] = dot4_add(G, B, Q[5]);
+    }
+    #pragma unroll
+    for (int k = 0; k < 3; k++) s[k] = small_u2f(S[k]);
+    #pragma unroll
+    for (int k = 0; k < 6; k++) s[3 + k] = small_u2f(Q[k]);
+}
+// a block's texels by channel: word r of x[c] holds channel c of row r
+__device__ __forceinline__ void block_by_channel(TexRef ts, uint4 x[3]) {
+    uint32_t w[4][4];
+    #pragma unroll
+    for (int r = 0; r < 4; r++) by_channel(ts[4 * r], ts[4 * r + 1], ts[4 * r + 2], ts[4 * r + 3], w[r]);
+    #pragma unroll
+    for (int c = 0; c < 3; c++) x[c] = make_uint4(w[0][c], w[1][c], w[2][c], w[3][c]);
+}
+
 // Mode 1's ranking of one opaque block (zap_tex.h:764-775) by the 8 lanes of a group (lane l, group mask gmask):
 // cand[0..3] the partitions of the four least (score, partition), -1 past the last valid one (group-uniform).
-// ts: the block's texels (the group's shared-memory copy).
+// ts: the block's texels (the group's shared-memory copy). Lane l scores partitions l, l + 8, ..., l + 56.
 __device__ __forceinline__ void group_rank(TexRef ts, int cand[kMode1Tries], const int l, const unsigned gmask) {
-    // ---- mode 1 ranking: lane scores partitions l, l + 8, ..., l + 56 (zap_tex.h:764-775), four per round:
-    // one pass over the texels adds each texel's 9 moments to the block totals and to the sums of the
-    // four partitions' subset 1, every sum in texel order as the reference adds them
-    float ce[kMode1Tries];
+    float ce[kMode1Tries], tot[9];
     int cp[kMode1Tries];
     #pragma unroll
     for (int j = 0; j < kMode1Tries; j++) { ce[j] = 1e30f; cp[j] = 64; }
+    uint4 x[3];
+    block_by_channel(ts, x);
+    subset_moments(x, 0xFFFFu, tot);
     #pragma unroll 1
-    for (int round = 0; round < 2; round++) {
-        uint32_t pm[4];
-        int n1[4];
-        float s1[4][9], tot[9];
+    for (int k = 0; k < 8; k++) {
+        const int part = l + kBc7Group * k;
+        const uint32_t pm = kP2[part];
+        float s1[9];
+        subset_moments(x, pm, s1);
+        const float e = partition_score(s1, __popc(pm), tot);
+        // insertion keeps (score, partition) order; NaN and >= 1e30 never enter, as in the reference
         #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            pm[k] = kP2[l + kBc7Group * (4 * round + k)];
-            n1[k] = 0;
-            #pragma unroll
-            for (int j = 0; j < 9; j++) s1[k][j] = 0.0f;
-        }
-        #pragma unroll
-        for (int j = 0; j < 9; j++) tot[j] = 0.0f;
-        #pragma unroll 1
-        for (int i = 0; i < 16; i++) {
-            const uint32_t x = ts[i];
-            const float rr = small_u2f(chan(x, 0)), gg = small_u2f(chan(x, 1)), bb = small_u2f(chan(x, 2));
-            const float mo[9] = {rr, gg, bb, rr * rr, gg * gg, bb * bb, rr * gg, rr * bb, gg * bb};
-            #pragma unroll
-            for (int j = 0; j < 9; j++) tot[j] = tot[j] + mo[j];
-            #pragma unroll
-            for (int k = 0; k < 4; k++)
-                if ((pm[k] >> i) & 1u) {
-                    n1[k]++;
-                    #pragma unroll
-                    for (int j = 0; j < 9; j++) s1[k][j] = s1[k][j] + mo[j];
-                }
-        }
-        #pragma unroll 1
-        for (int k = 0; k < 4; k++) {  // rolled: partition k's sums are at [0], the later ones shift down after it
-            const int part = l + kBc7Group * (4 * round + k);
-            const float e = partition_score(s1[0], n1[0], tot);
-            #pragma unroll
-            for (int r = 0; r < 3; r++) {
-                n1[r] = n1[r + 1];
+        for (int j = 0; j < kMode1Tries; j++) {
+            if (e < ce[j]) {
                 #pragma unroll
-                for (int j = 0; j < 9; j++) s1[r][j] = s1[r + 1][j];
-            }
-            // insertion keeps (score, partition) order; NaN and >= 1e30 never enter, as in the reference
-            #pragma unroll
-            for (int j = 0; j < kMode1Tries; j++) {
-                if (e < ce[j]) {
-                    #pragma unroll
-                    for (int s = kMode1Tries - 1; s > j; s--) { ce[s] = ce[s - 1]; cp[s] = cp[s - 1]; }
-                    ce[j] = e; cp[j] = part;
-                    break;
-                }
+                for (int s = kMode1Tries - 1; s > j; s--) { ce[s] = ce[s - 1]; cp[s] = cp[s - 1]; }
+                ce[j] = e; cp[j] = part;
+                break;
             }
         }
     }
@@ -590,23 +767,11 @@ __device__ __forceinline__ void cta_rank64(TexRef ts, int cand[kMode1Tries], flo
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t pm = kP2[tid];
     float s1[9], tot[9];
-    int n1 = 0;
-    #pragma unroll
-    for (int j = 0; j < 9; j++) { s1[j] = 0.0f; tot[j] = 0.0f; }
-    #pragma unroll 1
-    for (int i = 0; i < 16; i++) {
-        const uint32_t x = ts[i];
-        const float rr = small_u2f(chan(x, 0)), gg = small_u2f(chan(x, 1)), bb = small_u2f(chan(x, 2));
-        const float mo[9] = {rr, gg, bb, rr * rr, gg * gg, bb * bb, rr * gg, rr * bb, gg * bb};
-        #pragma unroll
-        for (int j = 0; j < 9; j++) tot[j] = tot[j] + mo[j];
-        if ((pm >> i) & 1u) {
-            n1++;
-            #pragma unroll
-            for (int j = 0; j < 9; j++) s1[j] = s1[j] + mo[j];
-        }
-    }
-    const float e = partition_score(s1, n1, tot);
+    uint4 x[3];
+    block_by_channel(ts, x);
+    subset_moments(x, 0xFFFFu, tot);
+    subset_moments(x, pm, s1);
+    const float e = partition_score(s1, __popc(pm), tot);
     const bool valid = e < 1e30f;  // NaN and >= 1e30 never enter, as in the reference
     float me = valid ? e : 1e30f;
     int mp = valid ? tid : 64;
@@ -628,6 +793,24 @@ __device__ __forceinline__ void cta_rank64(TexRef ts, int cand[kMode1Tries], flo
         if (bp < 64 && bp == tid) { me = 1e30f; mp = 64; }  // taken
         __syncthreads();  // the slots are written again next round
     }
+}
+
+// the mode-1 block (zap_tex.h:687-708) of a partition from each subset's endpoints (a: subset 0, b: subset 1; 6 bits a
+// channel, the p-bit in bit 18 of the first word) and the indices, 4 bits a texel, anchors already fixed
+__device__ __forceinline__ uint4 pack_mode1_block(int part, uint32_t a0, uint32_t a1, uint32_t b0w, uint32_t b1w, uint64_t full) {
+    Bits128 o;
+    o.put(2u, 2);
+    o.put((uint32_t)part, 6);
+    #pragma unroll
+    for (int c = 0; c < 3; c++) {
+        o.put((a0 >> (6 * c)) & 63u, 6); o.put((a1 >> (6 * c)) & 63u, 6);
+        o.put((b0w >> (6 * c)) & 63u, 6); o.put((b1w >> (6 * c)) & 63u, 6);
+    }
+    o.put((a0 >> 18) & 1u, 1); o.put((b0w >> 18) & 1u, 1);
+    const int anchor = (int)kA2[part];
+    #pragma unroll
+    for (int i = 0; i < 16; i++) o.put((uint32_t)((full >> (4 * i)) & 7u), (i == 0 || i == anchor) ? 2 : 3);
+    return make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]);
 }
 
 // Mode 1's fits of the ranked partitions cand[0..3] (-1: none) by the 8 lanes of a group, lane = candidate * 2 +
@@ -674,19 +857,7 @@ __device__ __forceinline__ bool mode1_fits(TexRef ts, const int cand[kMode1Tries
         int part = __shfl_sync(gmask, pj, 2 * bj, kBc7Group);
         err = (int)(ckey >> 2);
         uint64_t full = (uint64_t)il | ((uint64_t)ih << 32);
-        Bits128 o;
-        o.put(2u, 2);
-        o.put((uint32_t)part, 6);
-        #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            o.put((a0 >> (6 * c)) & 63u, 6); o.put((a1 >> (6 * c)) & 63u, 6);
-            o.put((b0w >> (6 * c)) & 63u, 6); o.put((b1w >> (6 * c)) & 63u, 6);
-        }
-        o.put((a0 >> 18) & 1u, 1); o.put((b0w >> 18) & 1u, 1);
-        const int anchor = (int)kA2[part];
-        #pragma unroll
-        for (int i = 0; i < 16; i++) o.put((uint32_t)((full >> (4 * i)) & 7u), (i == 0 || i == anchor) ? 2 : 3);
-        blk = make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]);
+        blk = pack_mode1_block(part, a0, a1, b0w, b1w, full);
         return true;
     }
     return false;
@@ -778,6 +949,286 @@ __device__ __forceinline__ int m5_alpha_lane(TexRef ts, int rot, uint32_t &qw, u
     return e5;
 }
 
+// ---------------------------------------------------------------- short lists: a CTA of 64 threads per listed block
+// While the list has no more blocks than the launch CTAs, each CTA takes one block and spreads it over its threads: as one
+// lane per mode-5 part and one 8-lane group for mode 1, the block was one chain of 53 k cycles (27 us; half of it mode 1's
+// fits). Eight threads share a mode-5 part (warp 0: the colour parts of the four rotations, warp 1: the alpha
+// parts) and then a mode-1 subset, as in mode6_encode_group: thread j has channel j & 3 of endpoint j >> 2 and two texels.
+struct HardBlock {
+    uint32_t px[16];   // the block's texels
+    uint4 ch[4];       // and by channel, a byte per texel
+    int cerr[4], aerr[4];
+    uint32_t cq[4], cq2[4], ci[4], aq[4], ai[4];  // per rotation, as pack_mode5_block takes them
+    int e1[8];                                     // per candidate and subset: mode 1's SSE, endpoints and indices
+    uint32_t w0[8], w1[8], ilo[8], ihi[8];
+    float re[2];
+    int rp[2];
+};
+struct RotRef {  // the texels as a mode-5 colour part has them
+    const uint32_t *p;
+    int rot;
+    __device__ __forceinline__ uint32_t operator[](int i) const { return rotate_texel(p[i], rot) & 0x00FFFFFFu; }
+};
+// the part's quantised endpoint value (m5_quant), q and x8
+template <int KIND>
+__device__ __forceinline__ int m5_part_group(HardBlock &H, int rot, uint32_t q[2], uint32_t &idx) {
+    constexpr bool kAlpha = KIND == kPartAlpha;
+    constexpr int kBits = kAlpha ? 8 : 7;
+    const int j = threadIdx.x & 7, c = kAlpha ? 0 : min(j & 3, 2), end = j >> 2, base = threadIdx.x & 31 & ~7;
+    const bool own = kAlpha ? (j & 3) == 0 : (j & 3) < 3;  // the thread whose value counts for (channel, endpoint)
+    const int i0 = 4 * (j & 3) + 2 * end;
+    uint32_t p[2];
+    #pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const uint32_t t = rotate_texel(H.px[i0 + i], rot);
+        p[i] = kAlpha ? t >> 24 : t & 0x00FFFFFFu;
+    }
+    const uint4 cw = H.ch[kAlpha ? (rot ? rot - 1 : 3) : (c == rot - 1 ? 3 : c)];
+    const uint32_t x4[4] = {cw.x, cw.y, cw.z, cw.w};
+    const uint32_t SX = dot4_add(x4[3], 0x01010101u, dot4_add(x4[2], 0x01010101u, dot4_add(x4[1], 0x01010101u, dot4(x4[0], 0x01010101u))));
+    const int pp = (int)(dot4(p[0], p[0]) + dot4(p[1], p[1]));
+    float v;
+    if (kAlpha) {  // the start: the range of the values
+        uint32_t lo = min(p[0], p[1]), hi = max(p[0], p[1]);
+        #pragma unroll
+        for (int m = 1; m < 8; m <<= 1) { lo = min(lo, __shfl_xor_sync(kAllLanes, lo, m)); hi = max(hi, __shfl_xor_sync(kAllLanes, hi, m)); }
+        v = small_u2f(end ? hi : lo);
+    } else {  // the principal axis
+        float mu[3], ax[3], n2 = 0.0f, tl = 1e9f, th = -1e9f;
+        pca_axis<3, 1>(RotRef{H.px, rot}, mu, ax);
+        #pragma unroll
+        for (int k = 0; k < 3; k++) n2 = n2 + ax[k] * ax[k];
+        #pragma unroll
+        for (int i = 0; i < 2; i++) {
+            float s = 0.0f;
+            #pragma unroll
+            for (int k = 0; k < 3; k++) s = s + (texel_at_2p15(p[i], k) - (mu[k] + 32768.0f)) * ax[k];
+            if (s < tl) tl = s;
+            if (s > th) th = s;
+        }
+        #pragma unroll
+        for (int m = 1; m < 8; m <<= 1) {
+            tl = fminf(tl, __shfl_xor_sync(kAllLanes, tl, m));
+            th = fmaxf(th, __shfl_xor_sync(kAllLanes, th, m));
+        }
+        const float muc = c == 0 ? mu[0] : c == 1 ? mu[1] : mu[2], axc = c == 0 ? ax[0] : c == 1 ? ax[1] : ax[2];
+        v = muc + axc * (end ? th : tl) / n2;
+    }
+    int err = 0;
+    q[0] = q[1] = 0u;
+    idx = 0u;
+    bool go = true;
+    #pragma unroll 1
+    for (int it = 0; it < 3; it++) {
+        if (it > 0) {
+            go = go && err > 0;
+            if (!__any_sync(kAllLanes, go)) break;
+            uint32_t W1 = 0u, W2 = 0u, SB = 0u;
+            #pragma unroll
+            for (int r = 0; r < 4; r++) {
+                uint32_t k = (idx >> (8 * r)) & 0xFFu;
+                k = (k | (k << 12)) & 0x000F000Fu;
+                k = (k | (k << 6)) & 0x03030303u;
+                const uint32_t K = 21u * k + ((k >> 1) & 0x01010101u);
+                W1 = dot4_add(K, 0x01010101u, W1); W2 = dot4_add(K, K, W2); SB = dot4_add(x4[r], K, SB);
+            }
+            const float aa = small_u2f(65536u - 128u * W1 + W2) * (1.0f / 4096.0f), ab = small_u2f(64u * W1 - W2) * (1.0f / 4096.0f);
+            const float bb = small_u2f(W2) * (1.0f / 4096.0f), det = aa * bb - ab * ab;
+            go = go && !(det < 1e-6f && det > -1e-6f);
+            const float sa = small_u2f(64u * SX - SB) * (1.0f / 64.0f), sb = small_u2f(SB) * (1.0f / 64.0f);
+            const float nv = clamp255((end ? sb * aa - sa * ab : sa * bb - sb * ab) / det);
+            v = go ? nv : 0.0f;
+        }
+        int tq, tx;
+        m5_quant1(v, kBits, tq, tx);
+        const uint32_t word = own ? (uint32_t)tq << (7 * c) : 0u;
+        const uint32_t n0 = or8(end ? 0u : word), n1 = or8(end ? word : 0u);
+        if (it > 0) {
+            go = go && !(n0 == q[0] && n1 == q[1]);
+            if (!__any_sync(kAllLanes, go)) break;
+        }
+        int x0[3], x1[3];
+        #pragma unroll
+        for (int k = 0; k < 3; k++) {
+            x0[k] = kAlpha ? (int)n0 : expand_bits((int)((n0 >> (7 * k)) & 127u), 7);
+            x1[k] = kAlpha ? (int)n1 : expand_bits((int)((n1 >> (7 * k)) & 127u), 7);
+        }
+        uint32_t pal[4];
+        int A[4];
+        m5_palette<KIND>(x0, x1, pal, A);
+        int e = pp;
+        uint32_t bits = 0u;
+        #pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int m = min(min(A[0] - 8 * (int)dot4(p[i], pal[0]), A[1] - 8 * (int)dot4(p[i], pal[1])),
+                              min(A[2] - 8 * (int)dot4(p[i], pal[2]), A[3] - 8 * (int)dot4(p[i], pal[3])));
+            e += m >> 2;
+            bits |= (uint32_t)(m & 3) << (2 * (i0 + i));
+        }
+        e = add8(e);
+        const uint32_t ni = or8(bits);
+        go = go && (it == 0 || e < err);
+        if (go) { err = e; idx = ni; q[0] = n0; q[1] = n1; }
+    }
+    (void)base;
+    return err;
+}
+// one subset of a mode-1 candidate (pca_endpoints, subset_passes<3, 3>): q: 6 bits a channel, bit 18 of q[0] the p-bit
+__device__ __forceinline__ int mode1_subset_group(HardBlock &H, uint32_t mask, uint32_t q[2], uint32_t &ilo, uint32_t &ihi) {
+    const int j = threadIdx.x & 7, c = min(j & 3, 2), end = j >> 2, i0 = 4 * (j & 3) + 2 * end;
+    const bool own = (j & 3) < 3;
+    const uint32_t p[2] = {H.px[i0] & 0x00FFFFFFu, H.px[i0 + 1] & 0x00FFFFFFu};
+    const bool in[2] = {((mask >> i0) & 1u) != 0u, ((mask >> (i0 + 1)) & 1u) != 0u};
+    const uint4 cw = H.ch[c];
+    const uint32_t x4[4] = {cw.x, cw.y, cw.z, cw.w}, n = (uint32_t)__popc(mask);
+    float lo[4], hi[4];
+    pca_endpoints<3, 1>(TexRef{H.px, 1}, mask, lo, hi);
+    float v = end ? (c == 0 ? hi[0] : c == 1 ? hi[1] : hi[2]) : (c == 0 ? lo[0] : c == 1 ? lo[1] : lo[2]);
+    int err = 0;
+    q[0] = q[1] = ilo = ihi = 0u;
+    bool go = true;
+    #pragma unroll 1
+    for (int it = 0; it < 3; it++) {
+        if (it > 0) {
+            go = go && err > 0;
+            if (!__any_sync(kAllLanes, go)) break;
+            uint32_t W1 = 0u, W2 = 0u, SB = 0u, SX = 0u;
+            #pragma unroll
+            for (int r = 0; r < 4; r++) {
+                uint32_t k = ((r < 2 ? ilo : ihi) >> (16 * (r & 1))) & 0xFFFFu;
+                k = (k | (k << 8)) & 0x00FF00FFu;
+                k = (k | (k << 4)) & 0x0F0F0F0Fu;
+                const uint32_t K = 9u * k + ((k >> 2) & 0x01010101u), ones = (((mask >> (4 * r)) & 15u) * 0x00204081u) & 0x01010101u;
+                W1 = dot4_add(K, 0x01010101u, W1); W2 = dot4_add(K, K, W2);
+                SB = dot4_add(x4[r], K, SB); SX = dot4_add(x4[r], ones, SX);
+            }
+            const float aa = small_u2f(4096u * n - 128u * W1 + W2) * (1.0f / 4096.0f), ab = small_u2f(64u * W1 - W2) * (1.0f / 4096.0f);
+            const float bb = small_u2f(W2) * (1.0f / 4096.0f), det = aa * bb - ab * ab;
+            go = go && !(det < 1e-6f && det > -1e-6f);
+            const float sa = small_u2f(64u * SX - SB) * (1.0f / 64.0f), sb = small_u2f(SB) * (1.0f / 64.0f);
+            const float nv = clamp255((end ? sb * aa - sa * ab : sa * bb - sb * ab) / det);
+            v = go ? nv : 0.0f;
+        }
+        const float v4[4] = {v, 0.0f, 0.0f, 0.0f};
+        int q0[4], q1[4], x8[4], e0 = quant_pbit<1>(v4, 7, 0, q0, x8), e1 = quant_pbit<1>(v4, 7, 1, q1, x8);
+        e0 = add8(own ? e0 : 0); e1 = add8(own ? e1 : 0);
+        const uint32_t pb = e1 < e0 ? 1u : 0u;  // shared by the subset's endpoints
+        const uint32_t word = own ? (uint32_t)(pb ? q1[0] : q0[0]) << (6 * c) : 0u;
+        const uint32_t n0 = or8(end ? 0u : word) | (pb << 18), n1 = or8(end ? word : 0u);
+        if (it > 0) {
+            go = go && !(n0 == q[0] && n1 == q[1]);
+            if (!__any_sync(kAllLanes, go)) break;
+        }
+        int x0[4] = {0, 0, 0, 0}, x1[4] = {0, 0, 0, 0};
+        #pragma unroll
+        for (int k = 0; k < 3; k++) {
+            x0[k] = expand_bits((int)((((n0 >> (6 * k)) & 63u) << 1) | pb), 7);
+            x1[k] = expand_bits((int)((((n1 >> (6 * k)) & 63u) << 1) | pb), 7);
+        }
+        const Lerp4 row(x0, x1);
+        int m0 = (int)0x80000000, m1 = (int)0x80000000;  // minus the least keys
+        #pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const uint32_t e = row.at(w3(k)) & 0x00FFFFFFu;
+            const int a = (int)dot4(e, e) * 8 + k;
+            m0 = max(m0, (int)(dot4(p[0], e) << 4) - a);
+            m1 = max(m1, (int)(dot4(p[1], e) << 4) - a);
+        }
+        int e = 0;
+        uint32_t two = 0u;
+        if (in[0]) { e += (-m0 >> 3) + (int)dot4(p[0], p[0]); two |= (uint32_t)-m0 & 7u; }
+        if (in[1]) { e += (-m1 >> 3) + (int)dot4(p[1], p[1]); two |= ((uint32_t)-m1 & 7u) << 4; }
+        e = add8(e);
+        const uint32_t nl = or8(i0 < 8 ? two << (4 * i0) : 0u), nh = or8(i0 < 8 ? 0u : two << (4 * (i0 - 8)));
+        go = go && (it == 0 || e < err);
+        if (go) { err = e; ilo = nl; ihi = nh; q[0] = n0; q[1] = n1; }
+    }
+    return err;
+}
+
+// modes 5 and 1 of one listed block (zap_tex.h:659-784); every thread of the CTA calls it
+__device__ __forceinline__ void hard_block(const SrcU8 &src, int bw, int by0, const BlockOut &out, size_t b0, uint2 item, HardBlock &H) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = (int)item.x;
+    if (tid < 4) {
+        uint32_t t[4], x[4];
+        gather_row(src, b % bw, by0 + b / bw, tid, t);
+        by_channel(t[0], t[1], t[2], t[3], x);
+        #pragma unroll
+        for (int i = 0; i < 4; i++) { H.px[4 * tid + i] = t[i]; ((uint32_t *)&H.ch[i])[tid] = x[i]; }
+    }
+    __syncthreads();
+    const int rot = lane >> 3;
+    uint32_t q[2], idx;
+    if (warp == 0) {
+        const int e = m5_part_group<kPartColour>(H, rot, q, idx);
+        if ((lane & 7) == 0) {
+            if (idx & 2u) { const uint32_t s = q[0]; q[0] = q[1]; q[1] = s; idx = ~idx; }  // anchor MSB must be 0
+            H.cerr[rot] = e; H.ci[rot] = idx;
+            H.cq[rot] = q[0] | (q[1] << 21); H.cq2[rot] = q[1] >> 7;  // seven bits a channel, endpoint 0 first
+        }
+    } else {
+        const int e = m5_part_group<kPartAlpha>(H, rot, q, idx);
+        if ((lane & 7) == 0) {
+            if (idx & 2u) { const uint32_t s = q[0]; q[0] = q[1]; q[1] = s; idx = ~idx; }
+            H.aerr[rot] = e; H.ai[rot] = idx;
+            H.aq[rot] = q[0] | (q[1] << 8);
+        }
+    }
+    __syncthreads();
+    uint32_t key = 0xFFFFFFFFu;  // the best rotation: (SSE, rotation) lexicographic
+    #pragma unroll
+    for (int r = 0; r < 4; r++) key = min(key, ((uint32_t)(H.cerr[r] + H.aerr[r]) << 2) | (uint32_t)r);
+    const int brot = (int)(key & 3u), best5 = (int)(key >> 2);
+    const uint4 a4 = H.ch[3];
+    const bool opaque = (a4.x & a4.y & a4.z & a4.w) == 0xFFFFFFFFu;
+    const int err = min(best5, (int)item.y);
+    uint4 blk = make_uint4(0, 0, 0, 0);
+    bool store = best5 < (int)item.y;  // decoded SSE == fit SSE (see the file header)
+    if (store && tid == 0) blk = pack_mode5_block(brot, H.cq[brot], H.cq2[brot], H.ci[brot], H.aq[brot], H.ai[brot]);
+    if (opaque) {  // CTA-uniform
+        int cand[kMode1Tries];
+        cta_rank64(TexRef{H.px, 1}, cand, H.re, H.rp);
+        const int task = tid >> 3, sub = task & 1;
+        int pj = cand[0];
+        #pragma unroll
+        for (int k = 1; k < kMode1Tries; k++) if (k == task >> 1) pj = cand[k];
+        const uint32_t pm = pj >= 0 ? (uint32_t)kP2[pj] : 0xFF00u, mask = sub ? pm : (~pm & 0xFFFFu);
+        uint32_t ilo, ihi;
+        const int e = mode1_subset_group(H, mask, q, ilo, ihi);
+        if ((lane & 7) == 0) {
+            const int anchor = sub ? (int)kA2[max(pj, 0)] : 0;
+            if (((anchor < 8 ? ilo >> (4 * anchor) : ihi >> (4 * (anchor - 8))) & 4u) != 0u) {  // anchor MSB must be 0
+                const uint32_t s = q[0], keep = q[0] & (1u << 18);
+                q[0] = q[1] | keep; q[1] = s & 0x3FFFFu;
+                uint64_t sel = 0;
+                #pragma unroll
+                for (int i = 0; i < 16; i++) if ((mask >> i) & 1u) sel |= 7ull << (4 * i);
+                ilo ^= (uint32_t)sel; ihi ^= (uint32_t)(sel >> 32);
+            }
+            H.e1[task] = pj >= 0 ? e : 1 << 29;
+            H.w0[task] = q[0]; H.w1[task] = q[1]; H.ilo[task] = ilo; H.ihi[task] = ihi;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            int be = err, bj = -1;  // the first candidate of the least SSE below err
+            #pragma unroll
+            for (int k = 0; k < kMode1Tries; k++) {
+                const int e2 = H.e1[2 * k] + H.e1[2 * k + 1];
+                if (cand[k] >= 0 && e2 < be) { be = e2; bj = k; }
+            }
+            if (bj >= 0) {
+                int part = cand[0];
+                #pragma unroll
+                for (int k = 1; k < kMode1Tries; k++) if (k == bj) part = cand[k];
+                blk = pack_mode1_block(part, H.w0[2 * bj], H.w1[2 * bj], H.w0[2 * bj + 1], H.w1[2 * bj + 1],
+                                       (uint64_t)(H.ilo[2 * bj] | H.ilo[2 * bj + 1]) | ((uint64_t)(H.ihi[2 * bj] | H.ihi[2 * bj + 1]) << 32));
+                store = true;
+            }
+        }
+    }
+    if (store && tid == 0) put_block16(out, b0 + (size_t)b, blk);
+}
+
 __global__ void __launch_bounds__(64, ZTC_MINB_BC7_MODE5) bc7_hard_kernel(SrcU8 src, int bw, int by0, BlockOut out, size_t b0,
                                                         const uint32_t *__restrict__ count, uint2 *items) {
     __shared__ uint32_t s_tex[kHardBlocks][17];  // per block (padded: the groups of a warp hit distinct banks)
@@ -785,14 +1236,16 @@ __global__ void __launch_bounds__(64, ZTC_MINB_BC7_MODE5) bc7_hard_kernel(SrcU8 
     __shared__ int s_cerr[kHardBlocks][4], s_aerr[kHardBlocks][4];
     __shared__ uint32_t s_cq[kHardBlocks][4], s_cq2[kHardBlocks][4], s_ci[kHardBlocks][4], s_aq[kHardBlocks][4], s_ai[kHardBlocks][4];
     __shared__ int s_op[64], s_wcnt[2];          // pass 2: the list positions of a chunk's opaque blocks
-    __shared__ float s_re[2];                    // cta_rank64's slots
-    __shared__ int s_rp[2];
+    __shared__ HardBlock s_one;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = (int)*(volatile const uint32_t *)count;
-    // one round per CTA at most (short lists): pass 2 finds the round's blocks in shared memory; one block per CTA at
-    // most (the shortest lists): that block's mode-1 ranking takes all 64 threads (these tests are grid-uniform)
-    const bool one_round = n <= (int)gridDim.x * kHardBlocks, sparse = n <= (int)gridDim.x;
-    const int per = sparse ? 1 : kHardBlocks;  // listed blocks per CTA and round
+    if (n <= (int)gridDim.x) {  // the shortest lists: one block per CTA at most (grid-uniform)
+        if ((int)blockIdx.x < n) hard_block(src, bw, by0, out, b0, items[blockIdx.x], s_one);
+        return;
+    }
+    // one round per CTA at most (short lists): pass 2 finds the round's blocks in shared memory (grid-uniform)
+    const bool one_round = n <= (int)gridDim.x * kHardBlocks;
+    constexpr int per = kHardBlocks;  // listed blocks per CTA and round
     // ---- pass 1, mode 5 (zap_tex.h:659-684) of every listed block the CTA holds, `per` per round: warp 0 fits the
     // colour parts and warp 1 the alpha parts, lane = block * 4 + rotation; the block is stored when mode 5 wins, and
     // its list entry keeps its SSE so far and, in bit 31 of the index, whether it is opaque (mode 1 is next)
@@ -800,7 +1253,7 @@ __global__ void __launch_bounds__(64, ZTC_MINB_BC7_MODE5) bc7_hard_kernel(SrcU8 
         if (tid < kHardBlocks) {  // one thread per block gathers its texels (16-byte row loads)
             const int it = base + tid;
             uint2 item = make_uint2(0xFFFFFFFFu, 0u);
-            if (tid < per && it < n) {
+            if (it < n) {
                 item = items[it];
                 uint32_t t[16];
                 gather_block(src, (int)item.x % bw, by0 + (int)item.x / bw, t);
@@ -869,17 +1322,12 @@ __global__ void __launch_bounds__(64, ZTC_MINB_BC7_MODE5) bc7_hard_kernel(SrcU8 
         }
         for (int k = g; k - g < total; k += kHardBlocks) {  // group-uniform: rounds of one block per group
             uint2 item = make_uint2(0xFFFFFFFFu, 0u);
-            if (sparse) item = s_item[0];  // CTA-uniform
-            else if (one_round) item = s_item[k];
+            if (one_round) item = s_item[k];
             else if (k < total) item = items[s_op[k]];
-            bool go = item.x != 0xFFFFFFFFu && (item.x >> 31) != 0u;
-            const int slot = sparse ? 0 : g;
-            TexRef ts{s_tex[slot], 1};
+            const bool go = item.x != 0xFFFFFFFFu && (item.x >> 31) != 0u;
+            TexRef ts{s_tex[g], 1};
             int cand[kMode1Tries];
-            if (sparse) {
-                if (go) cta_rank64(ts, cand, s_re, s_rp);  // every thread of the CTA
-                go = go && g == 0;
-            } else if (go) {
+            if (go) {
                 if (!one_round) {
                     const int b = (int)(item.x & 0x7FFFFFFFu);
                     uint32_t t[16];
@@ -899,9 +1347,7 @@ __global__ void __launch_bounds__(64, ZTC_MINB_BC7_MODE5) bc7_hard_kernel(SrcU8 
 // the modes-5/1 launch over a work list of at most nblocks items
 cudaError_t launch_hard(const SrcU8 &src, int bw, int by0, int nblocks, const BlockOut &out, size_t b0, const uint32_t *count,
                         uint2 *items, cudaStream_t s) {
-    int ctas = (nblocks + kHardBlocks - 1) / kHardBlocks;
-    const int cap = ztc_sm_count() * 8;
-    ctas = ctas < cap ? ctas : cap;
+    const int cap = ztc_sm_count() * 8, ctas = nblocks < cap ? nblocks : cap;  // a list of at most that many blocks takes a CTA each
     bc7_hard_kernel<<<ctas, 64, 0, s>>>(src, bw, by0, out, b0, count, items);
     return cudaGetLastError();
 }

@@ -604,21 +604,6 @@ __device__ __forceinline__ uint2 bc4_encode_quad(const uint32_t t[4], int c, int
     return make_uint2(quad_or((uint32_t)all) | (uint32_t)a0 | ((uint32_t)a1 << 8), quad_or((uint32_t)(all >> 32)));
 }
 
-// row r of block (bx, by), clamped to the image
-__device__ __forceinline__ void gather_row(const SrcU8 &s, int bx, int by, int r, uint32_t t[4]) {
-    const int x0 = bx * 4, y = min(by * 4 + r, s.h - 1);
-    #pragma unroll
-    for (int i = 0; i < 4; i++) t[i] = 0u;
-    if (!ZTC_IN_BOUNDS(x0, s.w, 1) || !ZTC_IN_BOUNDS(by * 4, s.h, 1)) return;
-    if (s.vec16 && x0 + 3 < s.w) {
-        const uint4 v = ldg((const uint4 *)(s.base + (size_t)y * s.stride + (size_t)x0 * 4));
-        t[0] = v.x; t[1] = v.y; t[2] = v.z; t[3] = v.w;
-        return;
-    }
-    #pragma unroll
-    for (int i = 0; i < 4; i++) t[i] = load_texel(s, min(x0 + i, s.w - 1), y);
-}
-
 constexpr int kGroupBlocks = 16;  // blocks of a 128-thread CTA, eight threads each
 template <int FMT>
 __global__ void __launch_bounds__(8 * kGroupBlocks) bcn_group_kernel(SrcU8 src, int bw, int by0, int nblocks, BlockOut out, size_t b0) {

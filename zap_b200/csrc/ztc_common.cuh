@@ -407,6 +407,21 @@ ZTC_DEV void gather_block(const SrcU8 &s, int bx, int by, uint32_t t[16]) {
     }
 }
 
+// row r of block (bx, by), clamped to the image
+ZTC_DEV void gather_row(const SrcU8 &s, int bx, int by, int r, uint32_t t[4]) {
+    const int x0 = bx * 4, y = min(by * 4 + r, s.h - 1);
+    #pragma unroll
+    for (int i = 0; i < 4; i++) t[i] = 0u;
+    if (!ZTC_IN_BOUNDS(x0, s.w, 1) || !ZTC_IN_BOUNDS(by * 4, s.h, 1)) return;
+    if (s.vec16 && x0 + 3 < s.w) {
+        const uint4 v = ldg((const uint4 *)(s.base + (size_t)y * s.stride + (size_t)x0 * 4));
+        t[0] = v.x; t[1] = v.y; t[2] = v.z; t[3] = v.w;
+        return;
+    }
+    #pragma unroll
+    for (int i = 0; i < 4; i++) t[i] = load_texel(s, min(x0 + i, s.w - 1), y);
+}
+
 // The block's texels as the rolled per-texel loops read them: texel i at p[i * stride]. On the device this is a
 // shared-memory copy of the block, so those loops need not be unrolled over registers and the kernels' code stays
 // small enough for the instruction cache (fully unrolled 16-texel x 16-entry palette scans, inlined at several
