@@ -18,8 +18,7 @@
 // Minimum resident 128-thread CTAs per SM requested from the register allocator, per kernel (tuned on B200:
 // more resident warps hide the latency of these long dependent integer / float chains; see the ncu summaries).
 // Measured on 2048x2048 encodes (re-swept after the loops were rolled): bc7_mode6 0.120 -> 0.113 ms at 6 (85
-// registers; the small spill stays in L1), BC1 -1.2 % at 8, ASTC single-partition -4 % at 5, BC6H (texels staged in
-// shared memory) 0.383 -> 0.351 ms at 5 against 3; the batched BC7 mode-1 kernel (118 registers already allow 4
+// registers; the small spill stays in L1), BC1 -1.2 % at 8, ASTC single-partition -4 % at 5, BC6H 4 (bc6_fit); the batched BC7 mode-1 kernel (118 registers already allow 4
 // CTAs) gains nothing from more.
 #ifndef ZTC_MINB_BC7_MODE6
 #define ZTC_MINB_BC7_MODE6 6
@@ -48,7 +47,7 @@
 #define ZTC_MINB_ASTC_SINGLE 5
 #endif
 #ifndef ZTC_MINB_BC6H
-#define ZTC_MINB_BC6H 5
+#define ZTC_MINB_BC6H 4
 #endif
 
 // ---------------------------------------------------------------- bounds checks (the ZTC_CHECKS build)
@@ -269,7 +268,9 @@ ZTC_DEV void by_channel(uint32_t t0, uint32_t t1, uint32_t t2, uint32_t t3, uint
 }
 #ifdef __CUDA_ARCH__
 ZTC_DEV int max3i(int a, int b, int c) { return __vimax3_s32(a, b, c); }
+ZTC_DEV uint32_t min3u(uint32_t a, uint32_t b, uint32_t c) { return __vimin3_u32(a, b, c); }
 #else
+inline uint32_t min3u(uint32_t a, uint32_t b, uint32_t c) { return a < b ? (a < c ? a : c) : (b < c ? b : c); }
 inline int max3i(int a, int b, int c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
 #endif
 ZTC_DEV uint32_t dot4_add(uint32_t a, uint32_t b, uint32_t c) {
