@@ -146,3 +146,19 @@ def test_bc7_around_the_launch_rules(cuda_lib, oracle, size):
     img = np.where(kind == 0, wide, np.where(kind == 1, flat, near)).clip(0, 255).astype(np.uint8)
     img[..., 3] = np.where(kind[..., 0] % 3 == 0, 255, img[..., 3])
     assert np.array_equal(zap_b200.bc_encode_dev(torch.from_numpy(img).cuda(), zap_b200.BC7).cpu().numpy(), oracle.bc_encode(img, zap_b200.BC7))
+
+
+@pytest.mark.parametrize("fmt", [zap_b200.BC1, zap_b200.BC3, zap_b200.BC4, zap_b200.BC5, zap_b200.BC7])
+@pytest.mark.parametrize("rdo", [1.0, 30.0, 300.0])
+def test_rdo_chains_of_every_short_length(cuda_lib, oracle, fmt, rdo):
+    """Chains of 1 to 21 blocks (the loader works four blocks ahead, the window holds 16), and a longer one with repeats, flat
+    stretches and noise, so that every candidate kind and match distance wins somewhere."""
+    rng = np.random.default_rng(int(rdo) + fmt)
+    for n in list(range(1, 22)) + [150]:
+        pool = rng.integers(0, 256, (5, 4, 4, 4), dtype=np.uint8)
+        pool[0] = pool[0, 0, 0]
+        blocks = [pool[rng.integers(0, 5)] if rng.random() < 0.5 else
+                  (pool[0].astype(int) + rng.integers(-12, 13, (4, 4, 4))).clip(0, 255).astype(np.uint8) for _ in range(n)]
+        img = np.ascontiguousarray(np.concatenate(blocks, axis=1))
+        got = zap_b200.bc_encode_rdo_dev(torch.from_numpy(img).cuda(), fmt, rdo)
+        assert np.array_equal(got.cpu().numpy(), oracle.bc_encode(img, fmt, rdo=rdo)), (fmt, rdo, n)

@@ -10,8 +10,8 @@
 // Only that window makes the work serial. The base encodings do not depend on it, so the ordinary encoder kernels
 // write them for every block first, in parallel. The chain then runs as one CTA per call (or per band of block
 // rows: each band is its own call in the reference's banded callers; and per sub-block kind, whose chains are
-// independent): per block, 16-lane groups evaluate the candidates side by side, one lane per texel, and a
-// CTA-wide minimum of (cost, candidate order) picks the winner. That minimum is the
+// independent): per block, groups of lanes evaluate the candidates side by side, and a minimum of (cost, candidate
+// order) picks the winner. That minimum is the
 // reference's choice: its scan takes a candidate only if its cost is below the best so far (strict "<"), so it ends
 // on the first candidate of the lowest cost, and its early "skip if SSE >= best" never changes that, because
 // SSE + lambda * rate >= SSE in float arithmetic when lambda * rate >= 0 (finite lambda > 0: the entry points reject
@@ -40,27 +40,12 @@ __host__ __device__ constexpr Sub sub_of(int fmt, int s) {
                                 : Sub{kBc7, 0, 0, 0};
 }
 
-// ---- BC1 sub-block (zap_tex.h:52-94): u16 c0, u16 c1, 2-bit indices; 3 colours + transparent when c0 <= c1
-ZTC_DEV void bc1_entry(uint32_t c0, uint32_t c1, int force4, int k, int &r, int &g, int &b) {
-    int r0, g0, b0, r1, g1, b1;
-    unpack565(c0, r0, g0, b0); unpack565(c1, r1, g1, b1);
-    const bool four = force4 || c0 > c1;
-    if (k == 0) { r = r0; g = g0; b = b0; }
-    else if (k == 1) { r = r1; g = g1; b = b1; }
-    else if (k == 2) {
-        if (four) { r = (2 * r0 + r1 + 1) / 3; g = (2 * g0 + g1 + 1) / 3; b = (2 * b0 + b1 + 1) / 3; }
-        else { r = (r0 + r1 + 1) / 2; g = (g0 + g1 + 1) / 2; b = (b0 + b1 + 1) / 2; }
-    } else {
-        if (four) { r = (r0 + 2 * r1 + 1) / 3; g = (g0 + 2 * g1 + 1) / 3; b = (b0 + 2 * b1 + 1) / 3; }
-        else { r = g = b = 0; }
-    }
-}
 // ---- BC4 sub-block (zap_tex.h:172-196): u8 a0, u8 a1, 3-bit indices; 6 values + 0 and 255 when a0 <= a1
 ZTC_DEV int bc4_entry(int a0, int a1, int k) {
-    if (k == 0) return a0;
-    if (k == 1) return a1;
-    if (a0 > a1) return ((8 - k) * a0 + (k - 1) * a1 + 3) / 7;
-    return k < 6 ? ((6 - k) * a0 + (k - 1) * a1 + 2) / 5 : k == 6 ? 0 : 255;
+    // without branches on the entry (a warp's lanes build one each); the numerators are below 2^11
+    const uint32_t n7 = (uint32_t)((8 - k) * a0 + (k - 1) * a1 + 3), n5 = (uint32_t)((6 - k) * a0 + (k - 1) * a1 + 2);
+    const int six = k < 6 ? (int)(n5 / 5u) : k == 6 ? 0 : 255;
+    return k == 0 ? a0 : k == 1 ? a1 : a0 > a1 ? (int)(n7 / 7u) : six;
 }
 // ---- BC7 mode-6 blocks (zap_tex.h:529)
 ZTC_DEV bool is_mode6(uint64_t lo) { return (lo & 0x7Fu) == 0x40u; }
@@ -392,10 +377,16 @@ __global__ void __launch_bounds__(B7Chain<L>::kThreads, 1) rdo_bc7_chain_kernel(
 // |t|^2 + |p_k|^2 - 2 t.p_k with t.p_k one dp4a; BC4 its 8 values. Each chosen sub-block enters the window with its
 // palette and the loader builds each block's base palette two blocks ahead, so no candidate builds one.
 ZTC_DEV int palette_word(const Sub &S, uint64_t v, int k) {
-    if (S.type == kBc1) {
-        int r, g, b;
-        bc1_entry((uint32_t)(v & 0xFFFFu), (uint32_t)((v >> 16) & 0xFFFFu), S.force4, k & 3, r, g, b);
-        const uint32_t p = pack_rgb(r, g, b);
+    if (S.type == kBc1) {  // (zap_tex.h:52-94: 3 colours and transparent when c0 <= c1) without branches on the entry: the loader's lanes build one word each
+        const uint32_t c0 = (uint32_t)(v & 0xFFFFu), c1 = (uint32_t)((v >> 16) & 0xFFFFu);
+        const bool four = S.force4 || c0 > c1;
+        int a[3], b[3];
+        unpack565(c0, a[0], a[1], a[2]); unpack565(c1, b[0], b[1], b[2]);
+        const int e = k & 3, wa = e == 0 ? 6 : e == 1 ? 0 : four ? (e == 2 ? 4 : 2) : 3;  // sixths of the first endpoint
+        uint32_t p = 0;
+        #pragma unroll
+        for (int c = 0; c < 3; c++) p |= (uint32_t)((a[c] * wa + b[c] * (6 - wa) + (e < 2 ? 0 : four ? 2 : 3)) / 6) << (8 * c);
+        if (e == 3 && !four) p = 0;
         return k < 4 ? (int)p : (int)dot4(p, p);
     }
     return bc4_entry((int)(v & 0xFFu), (int)((v >> 8) & 0xFFu), k);
@@ -405,24 +396,31 @@ ZTC_DEV int palette_word(const Sub &S, uint64_t v, int k) {
 // One chain per CTA and sub-block kind, in two roles. The candidates of a block that do not involve the block
 // chosen just before it (the base, and every neighbour at distance j >= 2) depend only on decisions at least two
 // blocks back, so producer warps evaluate them one block ahead: while block b - 1 is being chosen, they compute
-// block b's candidates (SSE, fields, and the match masks against window distances 2..16) into shared memory. A
-// chooser warp then decides block b alone: it evaluates the three candidates of neighbour distance 1 itself, adds
-// each other candidate's distance-1 match bit, turns the masks into rates and keys for all 49, and takes the minimum
-// of (cost, candidate order) across its lanes. One barrier per block; no CTA-wide minimum. The 49 candidates are
-// evaluated by groups of 8 lanes, lane q taking texels 2q, 2q + 1 and window distances 2q + 1, 2q + 2. Producer
-// groups: 0-15 kind 0 (neighbour j = (group & 15) + 2: its endpoints, fitted indices), 16-31 kind 1 (these
-// endpoints, its indices), 32-47 kind 2 (the whole neighbour), the last group of each kind idle (it repeats j = 16
-// and keeps nothing), 48 the base; a last warp loads the blocks ahead, software-pipelined (block b + 2 stored while
-// block b + 3 is fetched into registers), so no warp waits for a global load inside a step. The two sub-blocks of a
+// block b's candidates (SSE, fields, and the match masks against window distances 2..16) into shared memory. The
+// chooser then decides block b alone: three warps evaluate the three candidates of neighbour distance 1, one kind
+// each, down to their costs (sub_near), while the deciding warp adds the distance-1 match bit to the 46 others and turns
+// their masks into costs; a named barrier over the four joins them, and the deciding warp takes the minimum of (cost,
+// candidate order). One barrier per block; no CTA-wide minimum. The producers' candidates are evaluated by groups of L
+// lanes, lane q taking 16 / L texels and as many window distances. Producer groups: 0-15 kind 0 (neighbour j =
+// (group & 15) + 2: its endpoints, fitted indices), 16-31 kind 1 (these endpoints, its indices), 32-47 kind 2 (the
+// whole neighbour), the last group of each kind idle (it repeats j = 16 and keeps nothing), 48 the base; a last warp
+// loads the blocks ahead (block b + 2 stored while block b + 4 is fetched into registers). The two sub-blocks of a
 // BC3 or BC5 block are independent chains (each looks only at its own fields of earlier blocks, with its own match
 // distances, zap_tex.h:1494-1501), so each runs in its own CTA (blockIdx.y) and writes its own 8 bytes of the blocks.
-// The chooser is three warps: one fits the distance-1 kind-0 candidate, one evaluates kinds 1 and 2 (the same code
-// path), and the deciding warp meanwhile turns the other 46 candidates into keys (they do not depend on the distance-1
-// results); a named barrier over the three joins them, and the deciding warp adds the three distance-1 keys and takes
-// the minimum. Phase timers (clock64, a scratch build) put the chooser's step at ~2,950 cycles per block with all
-// three roles in one warp (the fit and evaluation branches serialised, then two candidates' keys per lane).
-constexpr int kSubL = 8, kSubProducerWarps = 13, kSubFit = 13, kSubEval = 14, kSubDecide = 15, kSubLoader = 16,
-              kSubThreads = 17 * 32;
+//
+// What bounds a chain is the length of a step: with a 1021x767 BC3 texture in 8-row bands (2048 blocks a chain), 2100 cycles
+// a block, the deciding warp's two keys per lane 1400 of them, next to one warp for two distance-1 kinds (1230 after the
+// keys were shortened) and a loader that waited for its own load (1500). Now about 1350, producers, deciding warp and
+// loader within a tenth of each other: field sizes known at compile time (-4 %), costs without the next match
+// distances, distance-1 candidates on 16 lanes with one reduction or vote per sum and mask (-22 % more), a warp per kind
+// and loads two blocks ahead (-9 %), palettes without branches on the entry (-5 %): 2.375 -> 1.53 ms.
+// A chain's warps at L lanes per producer candidate: producers, then the deciding warp, the three distance-1 warps and the
+// loader. BC1 chains take 4 lanes, launches with a BC4 chain 8: 512x512 in 8-row bands BC1 0.726 / 0.757 ms at 4 / 8, BC3
+// 0.796 / 0.757.
+template <int L>
+struct SubRoles {
+    static constexpr int kProducers = (49 * L + 31) / 32, kDecide = kProducers, kNear = kDecide + 1, kLoader = kNear + 3, kThreads = (kLoader + 1) * 32;
+};
 
 struct SubCand {
     int e;
@@ -434,13 +432,13 @@ struct SubCand {
 // One candidate of chain block b on a group of 8 lanes (gm: the lanes that meet its collectives). kind -1: the base;
 // 0: neighbour j's endpoints with fitted indices; 1: the base's endpoints with neighbour j's indices; 2: the whole
 // neighbour j. Its window masks cover distances dlo..16 (up to b).
+template <bool bc1, int L>
 __device__ __forceinline__ SubCand sub_candidate(const Sub &S, int kind, int j, int b, int q, unsigned gm, int dlo,
                                                  const uint32_t (*s_tex)[16], const uint64_t *s_base, const int (*s_bpal)[8],
                                                  const uint64_t *ring, const int (*ring_pal)[8]) {
-    constexpr int T = 16 / kSubL;
-    const bool bc1 = S.type == kBc1;
-    const int nA = bc1 ? 4 : 2, slot = b % 3;
-    const uint64_t maskA = (1ull << (8 * nA)) - 1ull;
+    constexpr int T = 16 / L, nA = bc1 ? 4 : 2;
+    constexpr uint64_t maskA = (1ull << (8 * nA)) - 1ull;
+    const int slot = b % 3;
     uint32_t t[T];
     #pragma unroll
     for (int u = 0; u < T; u++) t[u] = s_tex[slot][q * T + u];
@@ -461,15 +459,16 @@ __device__ __forceinline__ SubCand sub_candidate(const Sub &S, int kind, int j, 
             #pragma unroll
             for (int u = 0; u < T; u++) {
                 const uint32_t tc = t[u] & 0xFFFFFFu;
-                int bk = 0, be = pn.x - 2 * (int)dot4(tc, (uint32_t)pe.x), sk;
-                sk = pn.y - 2 * (int)dot4(tc, (uint32_t)pe.y); if (sk < be) { be = sk; bk = 1; }
-                sk = pn.z - 2 * (int)dot4(tc, (uint32_t)pe.z); if (sk < be) { be = sk; bk = 2; }
-                sk = pn.w - 2 * (int)dot4(tc, (uint32_t)pe.w); if (n4 && sk < be) { be = sk; bk = 3; }
-                e += be + (int)dot4(tc, tc);
-                idx |= (uint32_t)bk << (2 * (q * T + u));
+                // 4 (|p|^2 - 2 t.p) + entry: its least is the first nearest entry
+                const int k0 = 4 * (pn.x - 2 * (int)dot4(tc, (uint32_t)pe.x)), k1 = 4 * (pn.y - 2 * (int)dot4(tc, (uint32_t)pe.y)) + 1;
+                const int k2 = 4 * (pn.z - 2 * (int)dot4(tc, (uint32_t)pe.z)) + 2, k3 = 4 * (pn.w - 2 * (int)dot4(tc, (uint32_t)pe.w)) + 3;
+                int m = min(min(k0, k1), k2);
+                if (n4) m = min(m, k3);
+                e += (m >> 2) + (int)dot4(tc, tc);
+                idx |= ((uint32_t)m & 3u) << (2 * (q * T + u));
             }
-            e = lsum<kSubL>(e, gm);
-            idx = lor<kSubL>(idx, gm);
+            e = lsum<L>(e, gm);
+            idx = lor<L>(idx, gm);
         } else {  // zap__bc1_eval with the base's or the neighbour's indices
             idx = (uint32_t)((kind == -1 ? base : nb) >> 32);
             #pragma unroll
@@ -478,7 +477,7 @@ __device__ __forceinline__ SubCand sub_candidate(const Sub &S, int kind, int j, 
                 const int k = (int)((idx >> (2 * (q * T + u))) & 3u);
                 e += P[4 + k] - 2 * (int)dot4(tc, (uint32_t)P[k]) + (int)dot4(tc, tc);
             }
-            e = lsum<kSubL>(e, gm);
+            e = lsum<L>(e, gm);
         }
         r.cand = (uint64_t)a | ((uint64_t)c << 16) | ((uint64_t)idx << 32);
         // a 3-colour block may not use index 3 (transparent); the base is never checked
@@ -493,19 +492,16 @@ __device__ __forceinline__ SubCand sub_candidate(const Sub &S, int kind, int j, 
             #pragma unroll
             for (int u = 0; u < T; u++) {
                 const int v = (int)chan(t[u], S.chan);
-                int bk = 0, be = (v - pv[0]) * (v - pv[0]);
+                int m = 0x7FFFFFFF;  // 8 squared distance + entry: its least is the first nearest entry
                 #pragma unroll
-                for (int k = 1; k < 8; k++) {
-                    const int d = v - pv[k];
-                    if (d * d < be) { be = d * d; bk = k; }
-                }
-                e += be;
-                part |= (uint32_t)bk << (3 * u);
+                for (int k = 0; k < 8; k++) m = min(m, (v - pv[k]) * (v - pv[k]) * 8 + k);
+                e += m >> 3;
+                part |= ((uint32_t)m & 7u) << (3 * u);
             }
-            e = lsum<kSubL>(e, gm);
+            e = lsum<L>(e, gm);
             // lane q's indices start at bit 3 q T: two 32-bit words of the 48
             const uint64_t mine = (uint64_t)part << (3 * q * T);
-            idx = ((uint64_t)lor<kSubL>((uint32_t)(mine >> 32), gm) << 32) | lor<kSubL>((uint32_t)mine, gm);
+            idx = ((uint64_t)lor<L>((uint32_t)(mine >> 32), gm) << 32) | lor<L>((uint32_t)mine, gm);
         } else {  // zap__bc4_eval
             idx = (kind == -1 ? base : nb) >> 16;
             #pragma unroll
@@ -513,7 +509,7 @@ __device__ __forceinline__ SubCand sub_candidate(const Sub &S, int kind, int j, 
                 const int d = (int)chan(t[u], S.chan) - P[(int)((idx >> (3 * (q * T + u))) & 7u)];
                 e += d * d;
             }
-            e = lsum<kSubL>(e, gm);
+            e = lsum<L>(e, gm);
         }
         r.cand = (uint64_t)a | ((uint64_t)c << 8) | (idx << 16);
     }
@@ -529,115 +525,199 @@ __device__ __forceinline__ SubCand sub_candidate(const Sub &S, int kind, int j, 
             mB |= (uint32_t)((w >> (8 * nA)) == (r.cand >> (8 * nA))) << (d - 1);
         }
     }
-    r.mA = lor<kSubL>(mA, gm);
-    r.mB = lor<kSubL>(mB, gm);
+    r.mA = lor<L>(mA, gm);
+    r.mB = lor<L>(mB, gm);
     return r;
 }
 
-__global__ void __launch_bounds__(kSubThreads, 1) rdo_sub_chain_kernel(SrcU8 src, int bw, int nby, int chain_rows, uint8_t *__restrict__ out,
-                                                                      int bs, Sub S0, Sub S1, float lambda) {
-    __shared__ uint64_t ring[kWindow];  // the sub-block of the last 16 chosen blocks, slot = block & 15
-    __shared__ __align__(16) int ring_pal[kWindow][8];  // their palettes (palette_word)
-    __shared__ __align__(16) uint32_t s_tex[3][16];  // block b in slot b % 3
-    __shared__ uint64_t s_base[3];
-    __shared__ __align__(16) int s_bpal[3][8];  // the base sub-block's palette
+// the rate of a candidate (zap__field_rate per field) and its cost's bits (non-negative floats order like them);
+// mA, mB: its match masks, complete; d0, d1: the current match distances (bits past the window's blocks are never set)
+template <bool bc1>
+__device__ __forceinline__ uint32_t sub_cost(int e, uint32_t mA, uint32_t mB, int d0, int d1, float lambda) {
+    constexpr float sizeA = bc1 ? 4.0f : 2.0f, sizeB = bc1 ? 4.0f : 6.0f, newA = bc1 ? 3.0f : 2.0f, newB = 3.0f;  // new: min(size, 3)
+    const float fa = ((mA >> (d0 - 1)) & 1u) ? 0.0f : mA ? newA : sizeA, fb = ((mB >> (d1 - 1)) & 1u) ? 0.0f : mB ? newB : sizeB;
+    return e >= 0 ? __float_as_uint((float)e + lambda * (fa + fb)) : ~0u;
+}
+
+// A candidate of neighbour distance 1 of chain block b on 16 lanes, one texel and one window distance each: the chain's
+// longest path runs through it, so its sums and masks are one reduction or vote each instead of shuffle trees (lanes 0-15 of
+// a warp, l the lane). Kinds as in sub_candidate; cost: see sub_cost.
+template <bool bc1>
+__device__ __forceinline__ void sub_near(const Sub &S, int kind, int b, int l, const uint32_t (*s_tex)[16], const uint64_t *s_base,
+                                         const int (*s_bpal)[8], const uint64_t *ring, const int (*ring_pal)[8], int d0, int d1, float lambda,
+                                         uint64_t &cand, uint32_t &cost, uint32_t &masks) {
+    constexpr int nA = bc1 ? 4 : 2;
+    constexpr uint64_t maskA = (1ull << (8 * nA)) - 1ull;
+    constexpr unsigned gm = 0xFFFFu;
+    const int slot = b % 3, d = l + 1;
+    const uint32_t t = s_tex[slot][l];
+    const uint64_t base = s_base[slot], nb = ring[(b - 1) & (kWindow - 1)], w = ring[(b - d) & (kWindow - 1)];
+    const bool own = kind == 1;
+    const int *P = own ? s_bpal[slot] : ring_pal[(b - 1) & (kWindow - 1)];
+    bool ok = b >= 1;
+    int e;
+    if (bc1) {
+        const uint32_t a = (uint32_t)((own ? base : nb) & 0xFFFFu), c = (uint32_t)(((own ? base : nb) >> 16) & 0xFFFFu), tc = t & 0xFFFFFFu;
+        uint32_t idx = (uint32_t)(nb >> 32);
+        if (kind == 0) {  // zap__bc1_fit
+            const int4 pe = *(const int4 *)P, pn = *(const int4 *)(P + 4);
+            const int k0 = 4 * (pn.x - 2 * (int)dot4(tc, (uint32_t)pe.x)), k1 = 4 * (pn.y - 2 * (int)dot4(tc, (uint32_t)pe.y)) + 1;
+            const int k2 = 4 * (pn.z - 2 * (int)dot4(tc, (uint32_t)pe.z)) + 2, k3 = 4 * (pn.w - 2 * (int)dot4(tc, (uint32_t)pe.w)) + 3;
+            int m = min(min(k0, k1), k2);
+            if (S.force4 || a > c) m = min(m, k3);
+            e = (m >> 2) + (int)dot4(tc, tc);
+            idx = __reduce_or_sync(gm, ((uint32_t)m & 3u) << (2 * l));
+        } else {  // zap__bc1_eval
+            const int k = (int)((idx >> (2 * l)) & 3u);
+            e = P[4 + k] - 2 * (int)dot4(tc, (uint32_t)P[k]) + (int)dot4(tc, tc);
+        }
+        cand = (uint64_t)a | ((uint64_t)c << 16) | ((uint64_t)idx << 32);
+        if (!S.force4 && a <= c && (idx & (idx >> 1) & 0x55555555u)) ok = false;  // index 3 is transparent there
+    } else {
+        const int v = (int)chan(t, S.chan);
+        const uint32_t ac = (uint32_t)(own ? base : nb) & 0xFFFFu;
+        uint64_t idx = nb >> 16;
+        if (kind == 0) {  // zap__bc4_fit
+            const int4 p0 = *(const int4 *)P, p1 = *(const int4 *)(P + 4);
+            const int pv[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+            int m = 0x7FFFFFFF;
+            #pragma unroll
+            for (int k = 0; k < 8; k++) m = min(m, (v - pv[k]) * (v - pv[k]) * 8 + k);
+            e = m >> 3;
+            const uint64_t mine = (uint64_t)((uint32_t)m & 7u) << (3 * l);
+            idx = ((uint64_t)__reduce_or_sync(gm, (uint32_t)(mine >> 32)) << 32) | __reduce_or_sync(gm, (uint32_t)mine);
+        } else {  // zap__bc4_eval
+            const int x = v - P[(int)((idx >> (3 * l)) & 7u)];
+            e = x * x;
+        }
+        cand = (uint64_t)ac | (idx << 16);
+    }
+    e = __reduce_add_sync(gm, e);
+    const uint32_t mA = __ballot_sync(gm, d <= b && (w & maskA) == (cand & maskA)) & 0xFFFFu;
+    const uint32_t mB = __ballot_sync(gm, d <= b && (w >> (8 * nA)) == (cand >> (8 * nA))) & 0xFFFFu;
+    masks = mA | (mB << 16);
+    cost = sub_cost<bc1>(ok ? e : -1, mA, mB, d0, d1, lambda);
+}
+
+struct SubShared {
+    uint64_t ring[kWindow];  // the sub-block of the last 16 chosen blocks, slot = block & 15
+    __align__(16) int ring_pal[kWindow][8];  // their palettes (palette_word)
+    __align__(16) uint32_t tex[3][16];  // block b in slot b % 3
+    uint64_t base[3];
+    __align__(16) int bpal[3][8];  // the base sub-block's palette
     // the candidates of block b by candidate order (0 the base, (j - 1) * 3 + kind + 1 the others), buffer b & 1
-    __shared__ uint64_t c_cand[2][49];
-    __shared__ uint64_t c_meta[2][49];  // SSE (bit 31 set: not allowed) | mA << 32 | mB << 48
-    const Sub S = blockIdx.y ? S1 : S0;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = tid & (kSubL - 1), grp = tid / kSubL;
+    uint64_t cand[2][49];
+    uint64_t meta[2][49];  // SSE (bit 31 set: not allowed) | mA << 32 | mB << 48
+    uint2 near_cost[3];    // the distance-1 candidates' costs and masks (mA | mB << 16)
+    int dist[2];           // the current match distances (zap_tex.h:234)
+};
+// the chain of one sub-block kind, whose field sizes are known at compile time (the CTA's kind is uniform)
+template <bool bc1, int L>
+__device__ __forceinline__ void sub_chain(SubShared &M, const Sub S, const SrcU8 &src, int bw, int nby, int chain_rows, uint8_t *__restrict__ out, int bs,
+                                          float lambda) {
+    using R = SubRoles<L>;
+    auto &ring = M.ring;
+    auto &ring_pal = M.ring_pal;
+    auto &s_tex = M.tex;
+    auto &s_base = M.base;
+    auto &s_bpal = M.bpal;
+    auto &c_cand = M.cand;
+    auto &c_meta = M.meta;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = tid & (L - 1), grp = tid / L;
     const int row0 = blockIdx.x * chain_rows, rows = min(chain_rows, nby - row0);
     if (rows <= 0) return;
     const int first = row0 * bw, count = rows * bw;
-    // the loader warp: lane i < 16 fetches texel i of a block, every lane its base sub-block
-    uint32_t r_tex = 0;
-    uint64_t r_base = 0;
-    auto fetch = [&](int gk) {
-        if (lane < 16) r_tex = load_texel(src, min((gk % bw) * 4 + (lane & 3), src.w - 1), min((gk / bw) * 4 + (lane >> 2), src.h - 1));
-        r_base = *(const uint64_t *)(out + (size_t)gk * bs + S.off);
+    // the loader warp: lane i < 16 fetches texel i of a block, every lane its base sub-block; a fetched block waits a whole
+    // step in registers before it is stored, so a load has that long to arrive
+    struct Fetched {
+        uint32_t tex;
+        uint64_t base;
     };
-    auto store = [&](int ns) {  // the fetched block into slot ns, with the base's palette
-        if (lane < 16) s_tex[ns][lane] = r_tex;
-        if (lane < 8) s_bpal[ns][lane] = palette_word(S, r_base, lane);
-        if (lane == 0) s_base[ns] = r_base;
+    int fx = 0, fy = 0;  // the block row and column of the next fetch
+    auto fetch = [&]() {
+        Fetched f{0u, 0ull};
+        if (lane < 16) f.tex = load_texel(src, min(fx * 4 + (lane & 3), src.w - 1), min((row0 + fy) * 4 + (lane >> 2), src.h - 1));
+        f.base = *(const uint64_t *)(out + (size_t)(first + fy * bw + fx) * bs + S.off);
+        if (++fx == bw) { fx = 0; fy++; }
+        return f;
     };
-    if (warp == kSubLoader) {
-        fetch(first);
-        store(0);
-        if (count > 1) fetch(first + 1);
+    auto store = [&](const Fetched &f, int ns) {  // the fetched block into slot ns, with the base's palette
+        if (lane < 16) s_tex[ns][lane] = f.tex;
+        if (lane < 8) s_bpal[ns][lane] = palette_word(S, f.base, lane);
+        if (lane == 0) s_base[ns] = f.base;
+    };
+    Fetched f0{0u, 0ull}, f1{0u, 0ull};  // the next two blocks to store
+    if (tid == 0) { M.dist[0] = 1; M.dist[1] = 1; }
+    if (warp == R::kLoader) {
+        store(fetch(), 0);
+        if (count > 1) f0 = fetch();
+        if (count > 2) f1 = fetch();
     }
     __syncthreads();
     // producers: kind and neighbour distance of the group (the idle groups repeat j = 16), which warps hold one kind
     const int pkind = grp < 48 ? grp >> 4 : grp == 48 ? -1 : -3, pj = min((grp & 15) + 2, 16);
     const bool pkeep = grp < 48 ? (grp & 15) < 15 : grp == 48;
-    const unsigned pgm = warp < 12 ? 0xFFFFFFFFu : 0xFFu << (lane & 24);
-    // the chooser's fields and rates
-    const bool bc1 = S.type == kBc1;
-    const int nA = bc1 ? 4 : 2, nB = bc1 ? 4 : 6;
-    const uint64_t maskA = (1ull << (8 * nA)) - 1ull;
-    const float newA = bc1 ? 3.0f : 2.0f, newB = 3.0f;  // min(size, 3)
-    int d0 = 1, d1 = 1;  // the chooser's current match distances (zap_tex.h:234)
+    const unsigned pgm = warp < 48 * L / 32 ? 0xFFFFFFFFu : ((1u << L) - 1u) << (lane & ~(L - 1));
+    constexpr int nA = bc1 ? 4 : 2;
+    constexpr uint64_t maskA = (1ull << (8 * nA)) - 1ull;
+    int d0 = 1, d1 = 1;  // the deciding warp's current match distances (zap_tex.h:234)
     for (int it = -1; it < count; it++) {
         const int b = it + 1;  // the producers' block
-        if (warp < kSubProducerWarps) {
+        if (warp < R::kProducers) {
             if (pkind >= -1 && b < count) {
-                const SubCand c = sub_candidate(S, pkind, pj, b, q, pgm, 2, s_tex, s_base, s_bpal, ring, ring_pal);
+                const SubCand c = sub_candidate<bc1, L>(S, pkind, pj, b, q, pgm, 2, s_tex, s_base, s_bpal, ring, ring_pal);
                 if (pkeep && q == 0) {
                     const int o = pkind < 0 ? 0 : (pj - 1) * 3 + pkind + 1;
                     c_cand[b & 1][o] = c.cand;
                     c_meta[b & 1][o] = (uint32_t)c.e | (c.ok ? 0u : 0x80000000u) | ((uint64_t)c.mA << 32) | ((uint64_t)c.mB << 48);
                 }
             }
-        } else if (warp == kSubFit || warp == kSubEval) {
-            // the candidates of neighbour distance 1 (block it - 1, chosen in the previous step): kind 0 on the fit
-            // warp's lanes 0-7, kinds 1 and 2 on the evaluation warp's lanes 0-7 and 8-15
+        } else if (warp >= R::kNear && warp < R::kNear + 3) {
+            // the candidates of neighbour distance 1 (block it - 1, chosen in the previous step), down to their costs: one
+            // kind per warp, on its lanes 0-15
             if (it >= 0) {
-                const int ck = warp == kSubFit ? 0 : 1 + (lane >> 3);
-                if (lane < (warp == kSubFit ? 8 : 16)) {
-                    const SubCand c = sub_candidate(S, ck, 1, it, q, warp == kSubFit ? 0xFFu : 0xFFFFu, 1, s_tex, s_base, s_bpal, ring, ring_pal);
-                    if (q == 0) {
-                        c_cand[it & 1][ck + 1] = c.cand;
-                        c_meta[it & 1][ck + 1] = (uint32_t)c.e | (c.ok ? 0u : 0x80000000u) | ((uint64_t)c.mA << 32) | ((uint64_t)c.mB << 48);
-                    }
+                const int ck = warp - R::kNear;
+                if (lane < 16) {
+                    uint64_t cand;
+                    uint32_t cost, masks;
+                    sub_near<bc1>(S, ck, it, lane, s_tex, s_base, s_bpal, ring, ring_pal, M.dist[0], M.dist[1], lambda, cand, cost, masks);
+                    if (lane == 0) { c_cand[it & 1][ck + 1] = cand; M.near_cost[ck] = make_uint2(cost, masks); }
                 }
-                asm volatile("bar.sync 1, 96;" ::: "memory");  // with the deciding warp
+                asm volatile("bar.sync 1, 128;" ::: "memory");  // with the deciding warp
             }
-        } else if (warp == kSubDecide) {
+        } else if (warp == R::kDecide) {
             if (it >= 0) {
                 const int cur = it, bi = cur & 1;
                 const uint64_t w1 = ring[(cur - 1) & (kWindow - 1)];  // the block chosen in the previous step
-                uint64_t best = ~0ull;
-                int bd0 = d0, bd1 = d1;
-                // candidate o's key (zap__field_rate per field, the window's distance-1 bits added for the candidates
-                // the producers evaluated), kept if below the lane's best
-                auto consider = [&](int o) {
+                // candidate o's cost, the window's distance-1 bits added to the producers' masks
+                auto consider = [&](int o, uint32_t &masks) -> uint32_t {
                     const uint64_t cand = c_cand[bi][o], meta = c_meta[bi][o];
-                    uint32_t mA = (uint32_t)(meta >> 32) & 0xFFFFu, mB = (uint32_t)(meta >> 48);
-                    if ((o == 0 || o > 3) && cur >= 1) {
-                        mA |= (uint32_t)((w1 & maskA) == (cand & maskA));
-                        mB |= (uint32_t)((w1 >> (8 * nA)) == (cand >> (8 * nA)));
-                    }
-                    float fa = (float)nA, fb = (float)nB;
-                    int nd0 = d0, nd1 = d1;
-                    if (d0 > 0 && d0 <= cur && ((mA >> (d0 - 1)) & 1u)) fa = 0.0f;
-                    else if (mA) { nd0 = __ffs((int)mA); fa = newA; }
-                    if (d1 > 0 && d1 <= cur && ((mB >> (d1 - 1)) & 1u)) fb = 0.0f;
-                    else if (mB) { nd1 = __ffs((int)mB); fb = newB; }
-                    const int e = (int)(uint32_t)meta;
-                    const uint64_t key = e >= 0 ? key_of((float)e + lambda * (fa + fb), o) : ~0ull;
-                    if (key < best) { best = key; bd0 = nd0; bd1 = nd1; }
+                    const uint32_t near_bits = cur < 1 ? 0u : (uint32_t)((w1 & maskA) == (cand & maskA)) | ((uint32_t)((w1 >> (8 * nA)) == (cand >> (8 * nA))) << 16);
+                    masks = (uint32_t)(meta >> 32) | near_bits;
+                    return sub_cost<bc1>((int)(uint32_t)meta, masks & 0xFFFFu, masks >> 16, d0, d1, lambda);
                 };
-                consider(lane == 0 ? 0 : lane + 3);  // the base and orders 4..34
-                if (lane + 35 < 49) consider(lane + 35);  // orders 35..48
-                asm volatile("bar.sync 1, 96;" ::: "memory");  // the distance-1 candidates are in
-                if (lane >= 1 && lane <= 3) consider(lane);
-                const int order = (int)(uint32_t)warp_min_redux(best);
-                const int src = order <= 3 ? order : order <= 34 ? order - 3 : order - 35;  // the lane that keyed it
-                d0 = __shfl_sync(0xFFFFFFFFu, bd0, src);
-                d1 = __shfl_sync(0xFFFFFFFFu, bd1, src);
+                uint32_t masks, order = lane == 0 ? 0u : (uint32_t)lane + 3u;  // the base and orders 4..34
+                uint32_t cost = consider((int)order, masks);
+                if (lane + 35 < 49) {  // orders 35..48
+                    uint32_t m2;
+                    const uint32_t c2 = consider(lane + 35, m2);
+                    if (c2 < cost) { cost = c2; masks = m2; order = (uint32_t)lane + 35u; }
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");  // the distance-1 candidates are in
+                if (lane >= 1 && lane <= 3) {  // orders 1..3
+                    const uint2 n = M.near_cost[lane - 1];
+                    if (n.x <= cost) { cost = n.x; masks = n.y; order = (uint32_t)lane; }
+                }
+                const uint32_t least = __reduce_min_sync(0xFFFFFFFFu, cost);
+                order = __reduce_min_sync(0xFFFFFFFFu, cost == least ? order : ~0u);
+                const int win = order <= 3u ? (int)order : order <= 34u ? (int)order - 3 : (int)order - 35;  // the lane that has it
+                masks = __shfl_sync(0xFFFFFFFFu, masks, win);
+                const uint32_t mA = masks & 0xFFFFu, mB = masks >> 16;
+                if (mA && !((mA >> (d0 - 1)) & 1u)) d0 = __ffs((int)mA);
+                if (mB && !((mB >> (d1 - 1)) & 1u)) d1 = __ffs((int)mB);
                 // the winner enters the window with its palette (the base's, or the neighbour's: with j = 16 the
                 // neighbour's slot is this one, and each lane rewrites its own word)
-                const int oc = order - 1, wkind = oc % 3, wj = oc / 3 + 1;
+                const int oc = (int)order - 1, wkind = oc % 3, wj = oc / 3 + 1;
                 const uint64_t wc = c_cand[bi][order];
                 if (lane < 8) {
                     const int *P = order == 0 || wkind == 1 ? s_bpal[cur % 3] : ring_pal[(cur - wj) & (kWindow - 1)];
@@ -645,15 +725,28 @@ __global__ void __launch_bounds__(kSubThreads, 1) rdo_sub_chain_kernel(SrcU8 src
                 }
                 if (lane == 0) {
                     ring[cur & (kWindow - 1)] = wc;
+                    M.dist[0] = d0; M.dist[1] = d1;
                     if (order != 0) *(uint64_t *)(out + (size_t)(first + cur) * bs + S.off) = wc;
                 }
             }
-        } else {  // the loader: block it + 2 (fetched the step before) to shared memory; fetch block it + 3
-            if (it + 2 < count) store((it + 2) % 3);
-            if (it + 3 < count) fetch(first + it + 3);
+        } else {  // the loader: block it + 2 to shared memory, block it + 4 fetched
+            if (it + 2 < count) {
+                store(f0, (it + 2) % 3);
+                f0 = f1;
+                if (it + 4 < count) f1 = fetch();
+            }
         }
         __syncthreads();
     }
+}
+
+template <int L>
+__global__ void __launch_bounds__(SubRoles<L>::kThreads, 1) rdo_sub_chain_kernel(SrcU8 src, int bw, int nby, int chain_rows, uint8_t *__restrict__ out,
+                                                                      int bs, Sub S0, Sub S1, float lambda) {
+    __shared__ SubShared M;
+    const Sub S = blockIdx.y ? S1 : S0;
+    if (S.type == kBc1) sub_chain<true, L>(M, S, src, bw, nby, chain_rows, out, bs, lambda);
+    else sub_chain<false, L>(M, S, src, bw, nby, chain_rows, out, bs, lambda);
 }
 
 }  // namespace
@@ -684,7 +777,9 @@ cudaError_t ztc_launch_rdo(int fmt, const ztc::SrcU8 &src, uint8_t *out, float l
         const int ns = ztc::sub_count(fmt), bs = fmt == ZTC_FMT_BC1 || fmt == ZTC_FMT_BC4 ? 8 : 16;
         const dim3 grid(chains, ns);
         if (fmt < ZTC_FMT_BC1 || fmt > ZTC_FMT_BC5) return cudaErrorInvalidValue;
-        ztc::rdo_sub_chain_kernel<<<grid, ztc::kSubThreads, 0, stream>>>(src, bw, nby, band_rows, out, bs, S0, S1, lambda);
+        // see SubRoles
+        if (fmt == ZTC_FMT_BC1) ztc::rdo_sub_chain_kernel<4><<<grid, ztc::SubRoles<4>::kThreads, 0, stream>>>(src, bw, nby, band_rows, out, bs, S0, S1, lambda);
+        else ztc::rdo_sub_chain_kernel<8><<<grid, ztc::SubRoles<8>::kThreads, 0, stream>>>(src, bw, nby, band_rows, out, bs, S0, S1, lambda);
         return cudaGetLastError();
     }
 }
