@@ -97,14 +97,10 @@ ZTC_DEV void pca_power(float C[NC][NC], float ax[NC]) {
         for (int b = 0; b < a; b++) C[a][b] = C[b][a];
     #pragma unroll
     for (int c = 0; c < NC; c++) ax[c] = 1.0f;
-    if (UNROLL == 1) {
-        #pragma unroll 1
-        for (int it = 0; it < 6; it++)
-            if (!pca_power_step<NC>(C, ax)) break;
-    } else {
-        for (int it = 0; it < 6; it++)
-            if (!pca_power_step<NC>(C, ax)) break;
-    }
+    constexpr int kSteps = UNROLL == 1 ? 1 : 6;
+    #pragma unroll kSteps
+    for (int it = 0; it < 6; it++)
+        if (!pca_power_step<NC>(C, ax)) break;
 }
 // mean and axis of a whole block
 template <int NC, int UNROLL, typename Tex>
