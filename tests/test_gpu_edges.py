@@ -162,3 +162,18 @@ def test_rdo_chains_of_every_short_length(cuda_lib, oracle, fmt, rdo):
         img = np.ascontiguousarray(np.concatenate(blocks, axis=1))
         got = zap_b200.bc_encode_rdo_dev(torch.from_numpy(img).cuda(), fmt, rdo)
         assert np.array_equal(got.cpu().numpy(), oracle.bc_encode(img, fmt, rdo=rdo)), (fmt, rdo, n)
+
+
+@pytest.mark.parametrize("size", [(1, 1), (10, 7), (132, 4), (576, 572), (576, 580)])
+@pytest.mark.parametrize("opaque", [True, False])
+def test_astc_around_the_launch_rule(cuda_lib, oracle, size, opaque):
+    """A warp per trial up to 20720 blocks (140 per SM of 148), one thread for all three above; opaque and transparent blocks in one
+    image (they take different configurations), flat, near-flat and wide ones."""
+    w, h = size
+    rng = np.random.default_rng(w * 3 + h)
+    bw, bh = (w + 3) // 4, (h + 3) // 4
+    kind = np.kron(rng.integers(0, 5, (bh, bw)), np.ones((4, 4), int))[:h, :w, None]
+    flat = np.kron(rng.integers(0, 256, (bh, bw, 4)), np.ones((4, 4, 1), int))[:h, :w]
+    img = np.where(kind == 0, flat, np.where(kind == 1, rng.integers(0, 256, (h, w, 4)), flat + rng.integers(-9, 10, (h, w, 4)))).clip(0, 255).astype(np.uint8)
+    img[..., 3] = 255 if opaque else np.where(kind[..., 0] % 2 == 0, 255, img[..., 3])
+    assert np.array_equal(zap_b200.astc_encode_dev(torch.from_numpy(img).cuda()).cpu().numpy(), oracle.astc_encode(img))

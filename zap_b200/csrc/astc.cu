@@ -697,6 +697,68 @@ __global__ void __launch_bounds__(128, ZTC_MINB_ASTC_SINGLE) astc_single_kernel(
     }
 }
 
+// The single-partition search for small launches: a warp per trial. A CTA of three warps takes 32 blocks; lane l of warp k
+// runs trial k of block l from the principal axis to the last refit, then warp 0 picks each block's first trial of least SSE
+// and packs it. With fewer blocks than threads to spare, a block's three trials one after another were the launch's
+// length.
+constexpr int kTrialBlocks = 32;
+// Blocks per SM up to which a launch takes a warp per trial. One thread's three trials / a warp per trial: 64x64 opaque 58.6 / 44.9
+// us, 256x256 61.0 / 46.7, 512x512 60.0 / 53.1, 724x724 67.1 / 79.3; with alpha 42.8 / 29.0, 44.8 / 30.3, 46.0 / 37.2, 54.0 / 56.5.
+constexpr int kTrialLimit = 140;
+__global__ void __launch_bounds__(3 * kTrialBlocks) astc_trial_kernel(SrcU8 src, int bw, int by0, int nblocks, uint8_t *__restrict__ out,
+                                                                      uint32_t *__restrict__ count, uint2 *__restrict__ items) {
+    __shared__ AstcSmem S;
+    __shared__ uint32_t s_tex[16][kTrialBlocks];
+    __shared__ uint64_t s_code[3][kTrialBlocks];
+    __shared__ uint4 s_wt[3][kTrialBlocks];
+    __shared__ int s_err[3][kTrialBlocks];
+    load_smem(S);
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5, bi = blockIdx.x * kTrialBlocks + lane;
+    const int b = min(bi, nblocks - 1);  // lanes past the last block repeat it and store nothing
+    for (int r = k; r < 4; r += 3) {
+        uint32_t t[4];
+        gather_row(src, b % bw, by0 + b / bw, r, t);
+        #pragma unroll
+        for (int i = 0; i < 4; i++) s_tex[4 * r + i][lane] = t[i];
+    }
+    __syncthreads();
+    const TexRef ts{&s_tex[0][lane], kTrialBlocks};
+    uint32_t alpha = 0xFFFFFFFFu;
+    #pragma unroll
+    for (int i = 0; i < 16; i++) alpha &= ts[i];
+    const bool opaque = (alpha >> 24) == 255u;
+    {
+        float lo[1][4], hi[1][4];
+        if (opaque) pca_endpoints<3, 1, false>(ts, 0xFFFFu, lo[0], hi[0]);
+        else pca_endpoints<4, 1, false>(ts, 0xFFFFu, lo[0], hi[0]);
+        const int cfg = opaque ? k : 3 + k;
+        int code[1][8], uv[1][8], err = 0;
+        uint32_t wt[4] = {0, 0, 0, 0};
+        astc_trial_codes<32, 1>(S, cfg, lo, hi, code, uv);
+        astc_passes<32, 1>(ts, S, cfg, opaque ? 3 : 4, 0u, 0, 4, code, uv, wt, err);
+        s_code[k][lane] = bytes8(code[0]); s_wt[k][lane] = make_uint4(wt[0], wt[1], wt[2], wt[3]); s_err[k][lane] = err;
+    }
+    __syncthreads();
+    if (k != 0) return;
+    int best = s_err[0][lane], bk = 0;  // the first trial of least SSE (zap_tex.h:1306-1318)
+    #pragma unroll
+    for (int q = 1; q < 3; q++) if (s_err[q][lane] < best) { best = s_err[q][lane]; bk = q; }
+    const uint64_t c = s_code[bk][lane];
+    const uint4 w = s_wt[bk][lane];
+    const uint32_t codes[4] = {(uint32_t)c, (uint32_t)(c >> 32), 0u, 0u}, wts[4] = {w.x, w.y, w.z, w.w};
+    if (bi < nblocks) store_block16(out + (size_t)b * 16, astc_pack<1>(S, opaque ? bk : 3 + bk, 0, codes, wts));
+    const bool hard = bi < nblocks && opaque && best > 16 * 3 * 4;  // zap_tex.h:1323
+    const unsigned ballot = __ballot_sync(0xFFFFFFFFu, hard);
+    if (ballot) {
+        const int leader = __ffs(ballot) - 1;
+        uint32_t base = 0;
+        if (lane == leader) base = atomicAdd(count, (uint32_t)__popc(ballot));
+        base = __shfl_sync(0xFFFFFFFFu, base, leader);
+        const int pos = (int)base + __popc(ballot & ((1u << lane) - 1u));
+        if (hard && ZTC_IN_BOUNDS(pos, nblocks, 7)) items[pos] = make_uint2((uint32_t)b, (uint32_t)best);
+    }
+}
+
 // 2-means on RGB (zap_tex.h:1263-1283): bit i set = texel i in cluster 1
 ZTC_DEV uint32_t two_means(const uint32_t t[16]) {
     int lo = 0, hi = 0, slo = (int)(chan(t[0], 0) + chan(t[0], 1) + chan(t[0], 2)), shi = slo;
@@ -1138,16 +1200,16 @@ cudaError_t ztc_launch_astc(const ztc::SrcU8 &src, int by0, int nby, uint8_t *ou
     if (nblocks <= 0) return cudaSuccess;
     uint32_t *count = (uint32_t *)scratch;
     uint2 *items = (uint2 *)((uint8_t *)scratch + 256);
+    const int sms = ztc_sm_count();
     cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     {
         ztc::TraceScope tr("astc_single", stream);
         ztc::trace_units(nblocks);
-        ztc::astc_single_kernel<<<(nblocks + 127) / 128, 128, 0, stream>>>(src, bw, by0, nblocks, out, count, items);
+        if (nblocks <= sms * ztc::kTrialLimit)
+            ztc::astc_trial_kernel<<<(nblocks + ztc::kTrialBlocks - 1) / ztc::kTrialBlocks, 3 * ztc::kTrialBlocks, 0, stream>>>(src, bw, by0, nblocks, out, count, items);
+        else ztc::astc_single_kernel<<<(nblocks + 127) / 128, 128, 0, stream>>>(src, bw, by0, nblocks, out, count, items);
     }
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int ctas = nblocks < sms * 8 ? nblocks : sms * 8;  // a list of at most that many blocks takes a CTA each
     ztc::TraceScope tr("astc_two_part", stream);
     ztc::trace_units_dev(count, stream);
