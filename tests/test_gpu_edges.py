@@ -177,3 +177,27 @@ def test_astc_around_the_launch_rule(cuda_lib, oracle, size, opaque):
     img = np.where(kind == 0, flat, np.where(kind == 1, rng.integers(0, 256, (h, w, 4)), flat + rng.integers(-9, 10, (h, w, 4)))).clip(0, 255).astype(np.uint8)
     img[..., 3] = 255 if opaque else np.where(kind[..., 0] % 2 == 0, 255, img[..., 3])
     assert np.array_equal(zap_b200.astc_encode_dev(torch.from_numpy(img).cuda()).cpu().numpy(), oracle.astc_encode(img))
+
+
+@pytest.mark.parametrize("size", [(1, 1), (5, 6), (66, 20), (688, 688), (688, 692)])
+@pytest.mark.parametrize("form", ["rgb16f", "rgba16f", "rgba32f"])
+def test_bc6h_around_the_launch_rule(cuda_lib, oracle, size, form):
+    """A warp per start up to 29600 blocks (200 per SM of 148), one thread for both above; every input form at full and lesser
+    alignment, smooth and wild blocks, negatives, NaN and infinities."""
+    w, h = size
+    rng = np.random.default_rng(w + h + len(form))
+    bw, bh = (w + 3) // 4, (h + 3) // 4
+    base = np.kron(2.0 ** rng.uniform(-12, 14, (bh, bw, 3)), np.ones((4, 4, 1)))[:h, :w]
+    img = np.ones((h, w, 4), np.float32)
+    img[..., :3] = base * (1 + rng.uniform(-0.2, 0.2, (h, w, 3)))
+    wild = rng.random((h, w)) < 0.02
+    img[wild, 0] = rng.choice(np.array([np.nan, np.inf, -np.inf, -3.0, 0.0, 1e-7, 7e4], np.float32), int(wild.sum()))
+    if form != "rgba32f":
+        with np.errstate(over="ignore"):
+            img = img.astype(np.float16).astype(np.float32)
+    want = oracle.bc6h_encode(np.ascontiguousarray(img))
+    t = torch.from_numpy(img if form == "rgba32f" else img.astype(np.float16))[..., : 3 if form == "rgb16f" else 4].contiguous().cuda()
+    for pad in (0, 1):  # the image one texel into wider rows
+        wide = torch.zeros(h, w + 2 * pad, t.shape[2], dtype=t.dtype, device="cuda")
+        wide[:, pad:pad + w] = t
+        assert np.array_equal(zap_b200.bc6h_encode_dev(wide[:, pad:pad + w]).cpu().numpy(), want), (size, form, pad)

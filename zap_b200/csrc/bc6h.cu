@@ -377,6 +377,65 @@ __device__ __forceinline__ uint4 bc6h_encode_cta(bool valid, int16_t (*s_t)[CTA]
     return bc6_pack(be0, be1, s_idx[st][tid]);
 }
 
+// half bits h of texel i, channel c, and its pre-finish value h * 64 / 31, to [(3 i + c) * stride]
+__device__ __forceinline__ void bc6_put(uint32_t h, int i, int c, int16_t *t, float *U, int stride) {
+    t[(3 * i + c) * stride] = (int16_t)h;
+    U[(3 * i + c) * stride] = div_small(small_u2f(h) * 64.0f, 31.0f, 0x1.084210p-5f);  // RN(1/31)
+}
+// Rows [first, first + ROWS) of block (bx, by) (bc6_put). A row inside the image is read in the widest words its
+// alignment allows (24 bytes of RGB halfs as three 8-byte words, RGBA halfs as two 16-byte words, RGBA floats as four):
+// 12 loads a block instead of 48 (2048x2048 RGB halfs 215.5 -> 202.3 us).
+template <int ROWS>
+__device__ __forceinline__ void bc6_load(const SrcHdr &src, int bx, int by, int first, int16_t *t, float *U, int stride) {
+    const int x0 = bx * 4;
+    const uintptr_t bits = (uintptr_t)src.base | (src.stride * (src.f32 ? 4u : 2u));
+    const bool wide = x0 + 3 < src.w && (bits & (src.channels == 3 ? 7u : 15u)) == 0;
+    #pragma unroll
+    for (int k = 0; k < ROWS; k++) {
+        const int r = first + k, y = min(by * 4 + r, src.h - 1);
+        const size_t off = (size_t)y * src.stride + (size_t)x0 * (size_t)src.channels;
+        if (wide && src.f32) {
+            #pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float4 v = __ldg((const float4 *)((const float *)src.base + off) + j);
+                bc6_put(f2h_unsigned(v.x), 4 * r + j, 0, t, U, stride);
+                bc6_put(f2h_unsigned(v.y), 4 * r + j, 1, t, U, stride);
+                bc6_put(f2h_unsigned(v.z), 4 * r + j, 2, t, U, stride);
+            }
+        } else if (wide && src.channels == 3) {
+            uint32_t w[6];
+            #pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const uint2 v = __ldg((const uint2 *)((const uint16_t *)src.base + off) + j);
+                w[2 * j] = v.x; w[2 * j + 1] = v.y;
+            }
+            #pragma unroll
+            for (int j = 0; j < 12; j++) bc6_put(half_to_unsigned((w[j >> 1] >> (16 * (j & 1))) & 0xFFFFu), 4 * r + j / 3, j % 3, t, U, stride);
+        } else if (wide) {
+            #pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const uint4 v = __ldg((const uint4 *)((const uint16_t *)src.base + off) + j);
+                #pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const uint32_t rg = q ? v.z : v.x, ba = q ? v.w : v.y;
+                    bc6_put(half_to_unsigned(rg & 0xFFFFu), 4 * r + 2 * j + q, 0, t, U, stride);
+                    bc6_put(half_to_unsigned(rg >> 16), 4 * r + 2 * j + q, 1, t, U, stride);
+                    bc6_put(half_to_unsigned(ba & 0xFFFFu), 4 * r + 2 * j + q, 2, t, U, stride);
+                }
+            }
+        } else {
+            #pragma unroll 1
+            for (int j = 0; j < 4; j++) {
+                const size_t o = (size_t)y * src.stride + (size_t)min(x0 + j, src.w - 1) * (size_t)src.channels;
+                #pragma unroll
+                for (int c = 0; c < 3; c++)
+                    bc6_put(src.f32 ? f2h_unsigned(__ldg((const float *)src.base + o + c)) : half_to_unsigned(__ldg((const unsigned short *)src.base + o + c)),
+                            4 * r + j, c, t, U, stride);
+            }
+        }
+    }
+}
+
 constexpr int kBc6hCta = 128;
 __global__ void __launch_bounds__(kBc6hCta, ZTC_MINB_BC6H) bc6h_kernel(SrcHdr src, int bw, int by0, int nblocks, uint8_t *__restrict__ out) {
     __shared__ int16_t s_t[48][kBc6hCta];  // column threadIdx.x: this thread's block, centred
@@ -386,25 +445,43 @@ __global__ void __launch_bounds__(kBc6hCta, ZTC_MINB_BC6H) bc6h_kernel(SrcHdr sr
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = b < nblocks;
     if (valid) {
-        const int bx = b % bw, by = by0 + b / bw;
-        #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            int x = min(bx * 4 + (i & 3), src.w - 1), y = min(by * 4 + (i >> 2), src.h - 1);
-            size_t off = (size_t)y * src.stride + (size_t)x * (size_t)src.channels;
-            #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const uint32_t h = src.f32 ? f2h_unsigned(__ldg((const float *)src.base + off + c))
-                                           : half_to_unsigned(__ldg((const unsigned short *)src.base + off + c));
-                s_t[3 * i + c][threadIdx.x] = (int16_t)h;
-                s_U[3 * i + c][threadIdx.x] = div_small(small_u2f(h) * 64.0f, 31.0f, 0x1.084210p-5f);  // h * 64 / 31; RN(1/31)
-            }
-        }
+        bc6_load<4>(src, b % bw, by0 + b / bw, 0, &s_t[0][threadIdx.x], &s_U[0][threadIdx.x], kBc6hCta);
         uint32_t ts;
         s_cw[threadIdx.x] = bc6_center(&s_t[0][threadIdx.x], kBc6hCta, ts);
         s_ts[threadIdx.x] = ts;
     }
     const uint4 blk = bc6h_encode_cta<kBc6hCta>(valid, s_t, s_U, s_cw, s_ts);
     if (valid) store_block16(out + (size_t)b * 16, blk);
+}
+
+// The search for small launches: a warp per start. A CTA of two warps takes 32 blocks; lane l of warp k runs start k of
+// block l through all its passes, then warp 0 packs the first start of least SSE. With fewer blocks than threads to spare,
+// the two starts one after another and their compaction were the launch's length.
+constexpr int kStartBlocks = 32;
+// Blocks per SM up to which a launch takes a warp per start. One thread's two starts / a warp per start: 64x64 49.7 / 28.5 us,
+// 256x256 45.2 / 26.4, 512x512 43.8 / 31.2, 724x724 49.0 / 48.3, 1024x1024 66.2 / 76.4.
+constexpr int kStartLimit = 200;
+__global__ void __launch_bounds__(2 * kStartBlocks) bc6h_start_kernel(SrcHdr src, int bw, int by0, int nblocks, uint8_t *__restrict__ out) {
+    __shared__ int16_t s_t[48][kStartBlocks];
+    __shared__ float s_U[48][kStartBlocks];
+    __shared__ uint64_t s_cw[kStartBlocks], s_ends[2][kStartBlocks], s_idx[2][kStartBlocks], s_err[2][kStartBlocks];
+    __shared__ uint32_t s_ts[kStartBlocks];
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5, bi = blockIdx.x * kStartBlocks + lane;
+    const int b = min(bi, nblocks - 1);  // lanes past the last block repeat it and store nothing
+    bc6_load<2>(src, b % bw, by0 + b / bw, 2 * k, &s_t[0][lane], &s_U[0][lane], kStartBlocks);
+    __syncthreads();
+    if (k == 0) s_cw[lane] = bc6_center(&s_t[0][lane], kStartBlocks, s_ts[lane]);
+    __syncthreads();
+    const HalfRef B{&s_t[0][lane], &s_U[0][lane], kStartBlocks, s_cw[lane], s_ts[lane]};
+    uint64_t st[2];
+    bc6_start_ends(B, st);
+    bc6_passes(B, k ? st[1] : st[0], 0, 4, &s_ends[k][lane], &s_idx[k][lane], &s_err[k][lane]);
+    __syncthreads();
+    if (k != 0 || bi >= nblocks) return;
+    const int best = s_err[1][lane] < s_err[0][lane] ? 1 : 0;
+    int be0[3], be1[3];
+    unpack_ends10(s_ends[best][lane], be0, be1);
+    store_block16(out + (size_t)b * 16, bc6_pack(be0, be1, s_idx[best][lane]));
 }
 
 }  // namespace ztc
@@ -415,6 +492,8 @@ cudaError_t ztc_launch_bc6h(const ztc::SrcHdr &src, int by0, int nby, uint8_t *o
     if (nblocks <= 0) return cudaSuccess;
     ztc::TraceScope tr("bc6h_encode", stream);
     ztc::trace_units(nblocks);
-    ztc::bc6h_kernel<<<(nblocks + 127) / 128, 128, 0, stream>>>(src, bw, by0, nblocks, out);
+    if (nblocks <= ztc_sm_count() * ztc::kStartLimit)
+        ztc::bc6h_start_kernel<<<(nblocks + ztc::kStartBlocks - 1) / ztc::kStartBlocks, 2 * ztc::kStartBlocks, 0, stream>>>(src, bw, by0, nblocks, out);
+    else ztc::bc6h_kernel<<<(nblocks + 127) / 128, 128, 0, stream>>>(src, bw, by0, nblocks, out);
     return cudaGetLastError();
 }
