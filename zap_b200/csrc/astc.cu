@@ -665,7 +665,8 @@ ZTC_DEV uint4 astc_pack(const AstcSmem &S, int cfg, int seed, const uint32_t cod
     return astc_pack<1>(S, cfg, seed, codes, wt);
 }
 
-__global__ void __launch_bounds__(128, ZTC_MINB_ASTC_SINGLE) astc_single_kernel(SrcU8 src, int bw, int by0, int nblocks, uint8_t *__restrict__ out,
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) astc_single_kernel(SrcU8 src, int bw, int by0, int nblocks, uint8_t *__restrict__ out,
                                                           uint32_t *__restrict__ count, uint2 *__restrict__ items) {
     __shared__ AstcSmem S;
     __shared__ uint32_t s_tex[16][128];  // column threadIdx.x: this thread's block
@@ -1208,7 +1209,9 @@ cudaError_t ztc_launch_astc(const ztc::SrcU8 &src, int by0, int nby, uint8_t *ou
         ztc::trace_units(nblocks);
         if (nblocks <= sms * ztc::kTrialLimit)
             ztc::astc_trial_kernel<<<(nblocks + ztc::kTrialBlocks - 1) / ztc::kTrialBlocks, 3 * ztc::kTrialBlocks, 0, stream>>>(src, bw, by0, nblocks, out, count, items);
-        else ztc::astc_single_kernel<<<(nblocks + 127) / 128, 128, 0, stream>>>(src, bw, by0, nblocks, out, count, items);
+        else if (nblocks <= sms * 4 * 128)  // one wave at 4 CTAs per SM, without spills: 1024x1024 86.3 -> 83.2 us
+            ztc::astc_single_kernel<4><<<(nblocks + 127) / 128, 128, 0, stream>>>(src, bw, by0, nblocks, out, count, items);
+        else ztc::astc_single_kernel<ZTC_MINB_ASTC_SINGLE><<<(nblocks + 127) / 128, 128, 0, stream>>>(src, bw, by0, nblocks, out, count, items);
     }
     const int ctas = nblocks < sms * 8 ? nblocks : sms * 8;  // a list of at most that many blocks takes a CTA each
     ztc::TraceScope tr("astc_two_part", stream);

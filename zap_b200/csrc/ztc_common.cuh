@@ -17,21 +17,22 @@
 
 // Minimum resident 128-thread CTAs per SM requested from the register allocator, per kernel (tuned on B200:
 // more resident warps hide the latency of these long dependent integer / float chains; see the ncu summaries).
-// Measured on 2048x2048 encodes (re-swept after the loops were rolled): bc7_mode6 0.120 -> 0.113 ms at 6 (85
-// registers; the small spill stays in L1), BC1 -1.2 % at 8, ASTC single-partition -4 % at 5, BC6H 4 (bc6_fit); the batched BC7 mode-1 kernel (118 registers already allow 4
-// CTAs) gains nothing from more.
+// Measured again after the kernels changed: BC7 mode 6 at 7 (73 registers; the batch of 64 textures 2119 -> 2106 us against
+// 6, 5 2142; single images the same at all three), batched mode 1 at 5 (2119 -> 2100 against no limit), mode 5 at 8 (10
+// 2133, 6 2240), BC1 / BC3 at 7 (8 spills: the batch 2147 -> 2118, 1024x1024 BC1 55.1 -> 54.4), BC6H 4 (see bc6_fit);
+// ASTC's single-partition kernel 5 (2048x2048 169.2 us, 4 174, 6 180) in launches of more than one wave, else 4.
 #ifndef ZTC_MINB_BC7_MODE6
-#define ZTC_MINB_BC7_MODE6 6
+#define ZTC_MINB_BC7_MODE6 7
 #endif
 #ifndef ZTC_MINB_BC7_HARD
-#define ZTC_MINB_BC7_HARD 1
+#define ZTC_MINB_BC7_HARD 5
 #endif
 // the mode-5 launches (single image and batch): resident 64-thread CTAs per SM
 #ifndef ZTC_MINB_BC7_MODE5
 #define ZTC_MINB_BC7_MODE5 8
 #endif
 #ifndef ZTC_MINB_BCN
-#define ZTC_MINB_BCN 8
+#define ZTC_MINB_BCN 7
 #endif
 #ifndef ZTC_MINB_BCN_BATCH
 #define ZTC_MINB_BCN_BATCH ZTC_MINB_BCN
