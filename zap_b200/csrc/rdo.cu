@@ -60,28 +60,35 @@ __device__ __forceinline__ uint64_t key_of(float cost, int order) { return ((uin
 // 16-31 kind 2 (its indices, refit endpoints), 32-47 kind 0 (the whole neighbour), 48 the base; a last warp loads the
 // blocks ahead, software-pipelined like the BC1 / BC4 chains' loader (its own warp, so its global loads hold no
 // candidate's minimum). Every chosen block enters the window with its decoded texels and, for mode 6, its palette
-// (with the entries' squared norms), indices and index weights, so no candidate decodes a block: kind 0 compares the
+// (with 16 |p|^2 + k for entry k), indices and index weights, so no candidate decodes a block: kind 0 compares the
 // texels with the stored decode, kind 1 searches the stored palette. The base encodings are decoded for every block
 // by a parallel pass before the chains. Kind 2's least-squares sums are exact in the reference's float accumulation
 // (weights k/64, texels integers: every partial sum is a multiple of 1/4096 below 2^17 of them), so they are integer
 // dot products (the weights and the texels' channels a byte per texel), scaled, which gives the same floats in any
 // order; its solve and quantisation are one (channel, endpoint) per lane, both p-bits.
+//
+// What bounds a chain is the length of a step, about 2200 cycles a block: kind 2 1900 of them, kind 1 1700, the others
+// 1350-1500, the window's update 300. 512x512 in 8-row bands: the nearest values per parity by rule, end points and the
+// first word gathered in two packed words instead of twelve exchanges, weights from the window (1531 -> 1395 us); the
+// winner's window entries computed before the minimum and its group in the key, palette keys stored ready to subtract
+// from (-> 1268); the collectives as below (-> 1213).
 
-// Collectives over a group of L lanes: gm names the lanes that meet the collective. Warps whose groups all run one
-// kind of candidate pass the whole warp (every group meets each collective at the same point); whole-warp masks
-// measured faster on B200 than each group passing its own (512x512 one chain: BC7 30.6 -> 28.3 ms, BC1 25.8 ->
-// 25.5 ms), and redux.sync for the group sums slower than shuffle trees (BC7 30.6 -> 47 ms). ZTC_RDO_MIN_REDUX
-// selects redux.sync (1) or an xor-shuffle tree (0) for the warp-wide key minimum.
+// Sums and ORs over a group of L lanes; gm: the lanes of the warp that meet them. In the BC7 chain that is every lane
+// (the groups past the base's repeat it and never win), a mask known at compile time (512x512 in 8-row bands 1268 ->
+// 1217 us, with one OR for both fields' match masks). In the BC1 / BC4 chains the idle groups do nothing: those two
+// changes there measured BC1 726 -> 736 us next to BC3 1531 -> 1509. redux.sync for the group sums measured slower than
+// shuffle trees (BC7 512x512 in one chain: 30.6 -> 47 ms). ZTC_RDO_MIN_REDUX selects redux.sync (1) or an xor-shuffle
+// tree (0) for the warp-wide key minimum (BC7 as above: 1217 / 1365 us).
 #ifndef ZTC_RDO_MIN_REDUX
 #define ZTC_RDO_MIN_REDUX 1
 #endif
-// sums and ORs over a group of L lanes (gm: the lanes that meet the collective)
-template <int L> __device__ __forceinline__ int lsum(int v, unsigned gm) {
+constexpr unsigned kAll = 0xFFFFFFFFu;
+template <int L> __device__ __forceinline__ int lsum(int v, unsigned gm = kAll) {
     #pragma unroll
     for (int m = L / 2; m >= 1; m >>= 1) v += __shfl_xor_sync(gm, v, m, L);
     return v;
 }
-template <int L> __device__ __forceinline__ uint32_t lor(uint32_t v, unsigned gm) {
+template <int L> __device__ __forceinline__ uint32_t lor(uint32_t v, unsigned gm = kAll) {
     #pragma unroll
     for (int m = L / 2; m >= 1; m >>= 1) v |= __shfl_xor_sync(gm, v, m, L);
     return v;
@@ -106,6 +113,13 @@ __device__ __forceinline__ uint64_t warp_min_redux(uint64_t k) {
 ZTC_DEV int sq4px(uint32_t a, int aa, uint32_t b) { return aa + (int)dot4(b, b) - 2 * (int)dot4(a, b); }
 ZTC_DEV uint32_t lerp_px(const int x0[4], const int x1[4], int w) {
     return pack_rgba(lerp64(x0[0], x1[0], w), lerp64(x0[1], x1[1], w), lerp64(x0[2], x1[2], w), lerp64(x0[3], x1[3], w));
+}
+// mode 6's first word from expanded endpoints, a byte per channel (the last bit of each byte is that endpoint's p-bit)
+ZTC_DEV uint64_t mode6_lo(uint32_t X0, uint32_t X1) {
+    const uint32_t a = (X0 >> 1) & 0x7F7F7F7Fu, b = (X1 >> 1) & 0x7F7F7F7Fu;
+    const uint32_t rb = (a & 0x00FF00FFu) | ((b & 0x00FF00FFu) << 7), ga = ((a >> 8) & 0x00FF00FFu) | (((b >> 8) & 0x00FF00FFu) << 7);
+    const uint32_t rg = (rb & 0xFFFFu) | ((ga & 0xFFFFu) << 14), ba = (rb >> 16) | ((ga >> 16) << 14);  // 28 bits each
+    return ((uint64_t)((rg >> 25) | (ba << 3) | (X0 << 31)) << 32) | ((rg << 7) | 0x40u);
 }
 // mode 6 bit layout: mode bits 0-6, R0 R1 G0 G1 B0 B1 A0 A1 (7 bits each) from bit 7, P0 bit 63, P1 bit 64, then
 // the indices (texel 0: 3 bits, the others 4) from bit 65
@@ -171,11 +185,12 @@ template <int L> struct B7Chain {  // kWc candidate warps, then the loader warp
 template <int L>
 __global__ void __launch_bounds__(B7Chain<L>::kThreads, 1) rdo_bc7_chain_kernel(SrcU8 src, int bw, int nby, int chain_rows, uint8_t *__restrict__ out,
                                                                                 const uint32_t *__restrict__ dec_base, float lambda) {
+    static_assert(L >= 8, "a lane per (channel, endpoint) of a least-squares candidate");
     constexpr int T = B7Chain<L>::T, kW = B7Chain<L>::kWc;
     __shared__ uint64_t ring[kWindow][2];       // the last 16 chosen blocks, slot = block & 15
     __shared__ uint32_t ring_dec[kWindow][16];  // their decoded texels
     __shared__ __align__(16) uint32_t ring_pal[kWindow][16];  // mode 6: their palettes
-    __shared__ __align__(16) int ring_pp[kWindow][16];        // and the entries' squared norms |p|^2
+    __shared__ __align__(16) int ring_pp[kWindow][16];        // and 16 |p|^2 + k for entry k
     __shared__ uint64_t ring_idx[kWindow];      // mode 6: their indices, 4 bits per texel
     __shared__ __align__(16) uint32_t ring_wp[kWindow][4];  // mode 6: their index weights w4(idx), a byte per texel
     __shared__ uint32_t s_tex[3][16], s_dbase[3][16];  // block cur in slot cur % 3, loaded two blocks ahead
@@ -186,9 +201,8 @@ __global__ void __launch_bounds__(B7Chain<L>::kThreads, 1) rdo_bc7_chain_kernel(
     __shared__ int s_dist[2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = tid & (L - 1), grp = tid / L;
     const bool loader = warp == kW;
-    const int kind = loader ? -2 : grp < 16 ? 1 : grp < 32 ? 2 : grp < 48 ? 0 : grp == 48 ? -1 : -3, j = (grp & 15) + 1;
-    // the warps of groups 0-47 hold one kind each and meet every collective together; the base's group has its own
-    const unsigned gm = warp < 48 * L / 32 ? 0xFFFFFFFFu : (((1u << L) - 1u) << (lane & ~(L - 1)));
+    // the warps of groups 0-47 hold one kind each; the groups from 48 on all evaluate the base, for group 48
+    const int kind = loader ? -2 : grp < 16 ? 1 : grp < 32 ? 2 : grp < 48 ? 0 : -1, j = (grp & 15) + 1;
     const int row0 = blockIdx.x * chain_rows, rows = min(chain_rows, nby - row0);
     if (rows <= 0) return;
     const int first = row0 * bw, count = rows * bw;
@@ -206,7 +220,8 @@ __global__ void __launch_bounds__(B7Chain<L>::kThreads, 1) rdo_bc7_chain_kernel(
         const int g = first + cur, slot = cur % 3, d0 = s_dist[0], d1 = s_dist[1];
         uint64_t key = ~0ull, clo = 0, chi = 0, cidx = 0;
         uint32_t dec[T];  // the candidate's decode of this lane's texels
-        int nd0 = 0, nd1 = 0, x0[4], x1[4];  // x0, x1: kind 2's refit endpoints, expanded
+        int nd0 = 0, nd1 = 0;
+        uint32_t pal[T], wt[T];  // entries q T + u of the candidate's mode-6 palette, and its texels' index weights
         const int r = (cur - j) & (kWindow - 1);
         if (kind >= -1) {
             uint32_t t[T];
@@ -219,14 +234,19 @@ __global__ void __launch_bounds__(B7Chain<L>::kThreads, 1) rdo_bc7_chain_kernel(
                 clo = s_base[slot][0]; chi = s_base[slot][1];
                 #pragma unroll
                 for (int u = 0; u < T; u++) { dec[u] = s_dbase[slot][q * T + u]; e += sq4px(t[u], tt[u], dec[u]); }
-                e = lsum<L>(e, gm);
+                e = lsum<L>(e);
                 cidx = mode6_idx_of(chi);
+                #pragma unroll
+                for (int u = 0; u < T; u++) { pal[u] = s_bpal[slot][q * T + u]; wt[u] = (uint32_t)w4((int)((cidx >> (4 * (q * T + u))) & 15u)); }
                 ok = true;
             } else if (kind == 0) {  // the whole neighbour (zap__bc7_err)
                 clo = ring[r][0]; chi = ring[r][1]; cidx = ring_idx[r];
                 #pragma unroll
-                for (int u = 0; u < T; u++) { dec[u] = ring_dec[r][q * T + u]; e += sq4px(t[u], tt[u], dec[u]); }
-                e = lsum<L>(e, gm);
+                for (int u = 0; u < T; u++) {
+                    dec[u] = ring_dec[r][q * T + u]; e += sq4px(t[u], tt[u], dec[u]);
+                    pal[u] = ring_pal[r][q * T + u]; wt[u] = ((const uint8_t *)ring_wp[r])[q * T + u];
+                }
+                e = lsum<L>(e);
                 ok = j <= cur;
             } else if (kind == 1) {  // its endpoints, best indices; texel 0 keeps to 0..7 (zap__bc7_fit6_idx)
                 const uint64_t nlo = ring[r][0], nhi = ring[r][1];
@@ -241,10 +261,10 @@ __global__ void __launch_bounds__(B7Chain<L>::kThreads, 1) rdo_bc7_chain_kernel(
                     for (int k4 = 0; k4 < 4; k4++) {
                         const uint4 pk = *(const uint4 *)&ring_pal[r][4 * k4];
                         const int4 pp = *(const int4 *)&ring_pp[r][4 * k4];
-                        kk[4 * k4 + 0] = 16 * (pp.x - 2 * (int)dot4(t[u], pk.x)) + 4 * k4 + 0;
-                        kk[4 * k4 + 1] = 16 * (pp.y - 2 * (int)dot4(t[u], pk.y)) + 4 * k4 + 1;
-                        kk[4 * k4 + 2] = 16 * (pp.z - 2 * (int)dot4(t[u], pk.z)) + 4 * k4 + 2;
-                        kk[4 * k4 + 3] = 16 * (pp.w - 2 * (int)dot4(t[u], pk.w)) + 4 * k4 + 3;
+                        kk[4 * k4 + 0] = pp.x - 32 * (int)dot4(t[u], pk.x);
+                        kk[4 * k4 + 1] = pp.y - 32 * (int)dot4(t[u], pk.y);
+                        kk[4 * k4 + 2] = pp.z - 32 * (int)dot4(t[u], pk.z);
+                        kk[4 * k4 + 3] = pp.w - 32 * (int)dot4(t[u], pk.w);
                     }
                     if (i == 0) {  // the anchor texel's index has 3 bits
                         #pragma unroll
@@ -257,9 +277,10 @@ __global__ void __launch_bounds__(B7Chain<L>::kThreads, 1) rdo_bc7_chain_kernel(
                     dec[u] = ring_pal[r][kk[0] & 15];
                     e += (kk[0] >> 4) + tt[u];
                     bits |= (uint64_t)(kk[0] & 15) << (4 * i);
+                    pal[u] = ring_pal[r][i]; wt[u] = (uint32_t)w4(kk[0] & 15);
                 }
-                e = lsum<L>(e, gm);
-                cidx = ((uint64_t)lor<L>((uint32_t)(bits >> 32), gm) << 32) | lor<L>((uint32_t)bits, gm);
+                e = lsum<L>(e);
+                cidx = ((uint64_t)lor<L>((uint32_t)(bits >> 32)) << 32) | lor<L>((uint32_t)bits);
                 clo = nlo; chi = mode6_hi((int)(nhi & 1u), cidx);
             } else {  // its indices, least-squares endpoints, each endpoint's own p-bit (zap__bc7_fit6_ep)
                 const uint64_t nlo = ring[r][0], nhi = ring[r][1];
@@ -282,61 +303,49 @@ __global__ void __launch_bounds__(B7Chain<L>::kThreads, 1) rdo_bc7_chain_kernel(
                 else v = ep ? (bx * aa - ax * ab) / det : (ax * bb - bx * ab) / det;
                 v = clamp255(v);
                 // zap__bc7q for this (channel, endpoint), 7 bits + p, for both p-bits
-                const float vv = div255(v) * 255.0f;  // v / 255 correctly rounded, without a division sequence
-                int bq[2], be[2];
-                #pragma unroll
-                for (int p = 0; p < 2; p++) {
-                    const int gq = f2i_x86((vv - (float)p) / 2.0f + 0.5f);
-                    bq[p] = 0; be[p] = 1 << 30;
-                    #pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        const int tq = clampi(around(gq, k), 0, 127);
-                        const float d = (float)((tq << 1) | p) - v;
-                        const int ek = f2i_x86(d * d);
-                        if (ek < be[p]) { be[p] = ek; bq[p] = tq; }
-                    }
-                }
+                uint32_t bq[2][4];
+                int be[2];
+                quant8_pbits<1>(&v, bq, be);
                 // each endpoint's errors over the four channels, both p-bits in one word (each below 2^16: a
                 // candidate lies within 2 of v); the endpoint keeps the p-bit of the smaller sum, p = 0 on ties
                 int s2 = be[0] | (be[1] << 16);
-                s2 += __shfl_xor_sync(gm, s2, 2, L);
-                s2 += __shfl_xor_sync(gm, s2, 4, L);
-                const int pbm = (s2 >> 16) < (s2 & 0xFFFF) ? 1 : 0, qm = pbm ? bq[1] : bq[0];
-                const int pb0 = __shfl_sync(gm, pbm, 0, L), pb1 = __shfl_sync(gm, pbm, 1, L);
-                uint64_t lo = 0x40u | ((uint64_t)pb0 << 63);
-                #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int q0 = __shfl_sync(gm, qm, 2 * c, L), q1 = __shfl_sync(gm, qm, 2 * c + 1, L);
-                    x0[c] = (q0 << 1) | pb0; x1[c] = (q1 << 1) | pb1;
-                    lo |= ((uint64_t)q0 << (7 + 14 * c)) | ((uint64_t)q1 << (14 + 14 * c));
-                }
+                s2 += __shfl_xor_sync(kAll, s2, 2, L);
+                s2 += __shfl_xor_sync(kAll, s2, 4, L);
+                const uint32_t pbm = (s2 >> 16) < (s2 & 0xFFFF) ? 1u : 0u, qm = (pbm ? bq[1][0] : bq[0][0]) & 127u;
+                // the expanded endpoints gathered a byte per channel: X0 the first, X1 the second
+                uint32_t X = ((qm << 1) | pbm) << (8 * ch);
+                X |= __shfl_xor_sync(kAll, X, 2, L);
+                X |= __shfl_xor_sync(kAll, X, 4, L);
+                const uint32_t Y = __shfl_xor_sync(kAll, X, 1, L), X0 = ep ? Y : X, X1 = ep ? X : Y;
+                const Lerp4 fit(X0, X1);
                 #pragma unroll
                 for (int u = 0; u < T; u++) {
-                    dec[u] = lerp_px(x0, x1, w4((int)((cidx >> (4 * (q * T + u))) & 15u)));
+                    wt[u] = ((const uint8_t *)ring_wp[r])[q * T + u];
+                    dec[u] = fit.at((int)wt[u]); pal[u] = fit.at(w4(q * T + u));
                     e += sq4px(t[u], tt[u], dec[u]);
                 }
-                e = lsum<L>(e, gm);
-                clo = lo; chi = (nhi & ~1ull) | (uint64_t)pb1;
+                const uint32_t pb1 = X1 & 1u;
+                const uint64_t lo = mode6_lo(X0, X1);
+                e = lsum<L>(e);
+                clo = lo; chi = (nhi & ~1ull) | pb1;
             }
             // rate (zap__bc7_rate): bit d - 1 of a mask says the field equals the window's at distance d
-            uint32_t mA = 0, mB = 0;
+            uint32_t m2 = 0;  // the two fields' masks in one word's halves
             #pragma unroll
             for (int u = 0; u < T; u++) {
                 const int d = q * T + u + 1, rw = (cur - d) & (kWindow - 1);
-                if (d <= cur) {
-                    mA |= (uint32_t)(ring[rw][0] == clo) << (d - 1);
-                    mB |= (uint32_t)((ring[rw][1] >> 8) == (chi >> 8)) << (d - 1);
-                }
+                if (d <= cur) m2 |= (((uint32_t)(ring[rw][0] == clo)) | ((uint32_t)((ring[rw][1] >> 8) == (chi >> 8)) << 16)) << (d - 1);
             }
-            mA = lor<L>(mA, gm);
-            mB = lor<L>(mB, gm);
+            m2 = lor<L>(m2);
+            const uint32_t mA = m2 & 0xFFFFu, mB = m2 >> 16;
             float fa = 8.0f, fb = 7.0f;
             nd0 = d0; nd1 = d1;
             if (d0 > 0 && d0 <= cur && ((mA >> (d0 - 1)) & 1u)) fa = 0.0f;
             else if (mA) { nd0 = __ffs((int)mA); fa = 3.0f; }
             if (d1 > 0 && d1 <= cur && ((mB >> (d1 - 1)) & 1u)) fb = 0.0f;
             else if (mB) { nd1 = __ffs((int)mB); fb = 3.0f; }
-            if (ok) key = key_of((float)e + lambda * (fa + fb + 1.0f), kind < 0 ? 0 : (j - 1) * 3 + kind + 1);
+            // the order, then the group that holds the candidate
+            if (ok) key = key_of((float)e + lambda * (fa + fb + 1.0f), (kind < 0 ? 0 : (j - 1) * 3 + kind + 1) << 8 | grp);
         } else if (loader) {  // block cur + 2 (fetched the iteration before) to shared memory; fetch block cur + 3
             if (cur + 2 < count) fb.store(lane, (cur + 2) % 3, s_tex, s_dbase, s_base, s_bpal, s_texc);
             if (cur + 3 < count) fb.fetch(src, bw, out, dec_base, g + 3, lane);
@@ -346,26 +355,21 @@ __global__ void __launch_bounds__(B7Chain<L>::kThreads, 1) rdo_bc7_chain_kernel(
             if (lane == 0) s_key[warp] = wk;
         }
         __syncthreads();
-        const int order = loader ? -1 : (int)(uint32_t)warp_min_redux(lane < kW ? s_key[lane] : ~0ull);
-        const int oc = order - 1, wkind = oc % 3, wgrp = order == 0 ? 48 : wkind == 1 ? oc / 3 : wkind == 2 ? 16 + oc / 3 : 32 + oc / 3;
-        if (!loader && grp == wgrp) {  // the winner enters the window
+        const int won = loader ? -1 : (int)((uint32_t)warp_min_redux(lane < kW ? s_key[lane] : ~0ull) & 0xFFu);
+        if (grp == won) {  // the winner enters the window (with j = 16 its slot is the one it read; all it writes was read before the barrier)
             const int ws = cur & (kWindow - 1);
-            // its decode, its mode-6 palette (the base's, built by the loader; the neighbour's, which kinds 0 and 1
-            // keep: with j = 16 that slot is this one and each lane rewrites its own entries; or from the refit
-            // endpoints) and its index weights
             #pragma unroll
             for (int u = 0; u < T; u++) {
                 const int i = q * T + u;
                 ring_dec[ws][i] = dec[u];
-                const uint32_t pal = order == 0 ? s_bpal[slot][i] : kind != 2 ? ring_pal[r][i] : lerp_px(x0, x1, w4(i));
-                ring_pal[ws][i] = pal;
-                ring_pp[ws][i] = (int)dot4(pal, pal);
-                ((uint8_t *)ring_wp[ws])[i] = (uint8_t)w4((int)((cidx >> (4 * i)) & 15u));
+                ring_pal[ws][i] = pal[u];
+                ring_pp[ws][i] = 16 * (int)dot4(pal[u], pal[u]) + i;
+                ((uint8_t *)ring_wp[ws])[i] = (uint8_t)wt[u];
             }
             if (q == 0) {
                 ring[ws][0] = clo; ring[ws][1] = chi; ring_idx[ws] = cidx;
                 s_dist[0] = nd0; s_dist[1] = nd1;
-                if (order != 0) { *(uint64_t *)(out + (size_t)g * 16) = clo; *(uint64_t *)(out + (size_t)g * 16 + 8) = chi; }
+                if (kind >= 0) { *(uint64_t *)(out + (size_t)g * 16) = clo; *(uint64_t *)(out + (size_t)g * 16 + 8) = chi; }
             }
         }
         __syncthreads();
@@ -429,7 +433,7 @@ struct SubCand {
     uint32_t mA, mB;  // bit d - 1: the field equals the window's at distance d (from distance dlo on)
 };
 
-// One candidate of chain block b on a group of 8 lanes (gm: the lanes that meet its collectives). kind -1: the base;
+// One candidate of chain block b on a group of L lanes (gm: the lanes that meet its collectives). kind -1: the base;
 // 0: neighbour j's endpoints with fitted indices; 1: the base's endpoints with neighbour j's indices; 2: the whole
 // neighbour j. Its window masks cover distances dlo..16 (up to b).
 template <bool bc1, int L>
@@ -656,8 +660,8 @@ __device__ __forceinline__ void sub_chain(SubShared &M, const Sub S, const SrcU8
     __syncthreads();
     // producers: kind and neighbour distance of the group (the idle groups repeat j = 16), which warps hold one kind
     const int pkind = grp < 48 ? grp >> 4 : grp == 48 ? -1 : -3, pj = min((grp & 15) + 2, 16);
+    const unsigned pgm = warp < 48 * L / 32 ? kAll : ((1u << L) - 1u) << (lane & ~(L - 1));
     const bool pkeep = grp < 48 ? (grp & 15) < 15 : grp == 48;
-    const unsigned pgm = warp < 48 * L / 32 ? 0xFFFFFFFFu : ((1u << L) - 1u) << (lane & ~(L - 1));
     constexpr int nA = bc1 ? 4 : 2;
     constexpr uint64_t maskA = (1ull << (8 * nA)) - 1ull;
     int d0 = 1, d1 = 1;  // the deciding warp's current match distances (zap_tex.h:234)

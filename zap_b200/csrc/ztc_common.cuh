@@ -179,6 +179,11 @@ struct Lerp4 {
         srb = (uint32_t)(x1[0] - x0[0]) + ((uint32_t)(x1[2] - x0[2]) << 16);  // modulo 2^32, as the sums are
         sga = (uint32_t)(x1[1] - x0[1]) + ((uint32_t)(x1[3] - x0[3]) << 16);
     }
+    ZTC_DEV Lerp4(uint32_t x0, uint32_t x1) {  // endpoints packed like texels
+        const uint32_t rb0 = x0 & 0x00FF00FFu, ga0 = (x0 >> 8) & 0x00FF00FFu;
+        rb = 64u * rb0 + 0x00200020u; ga = 64u * ga0 + 0x00200020u;
+        srb = (x1 & 0x00FF00FFu) - rb0; sga = ((x1 >> 8) & 0x00FF00FFu) - ga0;
+    }
     ZTC_DEV uint32_t at(int w) const {  // the four channels' lerp64 at weight w, as a texel
         const uint32_t a = rb + srb * (uint32_t)w, b = ga + sga * (uint32_t)w;
         return ((a >> 6) & 0x00FF00FFu) | ((b << 2) & 0xFF00FF00u);
