@@ -285,7 +285,7 @@ ZTC_DEV uint2 bc1_encode(const uint32_t t[16]) {
 // thread's block is in t and in column threadIdx.x of s_tex.
 // ROLLED: the starts' principal axis and least-squares sums run in rolled loops over s_tex (less code, more
 // instructions): faster in launches of several waves, slower in a launch of less than one wave, where each
-// thread's own chain of dependent instructions sets the time (512x512 BC1: 0.0415 -> 0.0441 ms).
+// thread's own chain of dependent instructions sets the time (512x512 BC1, one thread per block: 0.0415 -> 0.0441 ms).
 template <int CTA, bool ROLLED>
 __device__ __forceinline__ uint2 bc1_encode_cta(bool valid, const uint32_t t[16], uint32_t (*s_tex)[CTA]) {
     static_assert(CTA % 32 == 0 && CTA <= 256, "whole warps, owners fit a byte");
