@@ -173,10 +173,11 @@ __device__ __forceinline__ MipSource mip_load(const MipChain &C, int tx, int ty)
     return m;
 }
 
-// Tile (tx, ty) of one chain: levels 1..C.levels below its 64x64 source texels m; n counts the CTA's tiles. Every
-// thread of the CTA calls it. Levels 3..6 of tile n are one warp's work (warp n modulo 8) while the others go on to
-// the next tile, so a tile has one barrier: S[n & 1] is written again two tiles on, after a barrier that this
-// tile's warp reaches only when it is done.
+// Tile (tx, ty) of one chain: levels 1..C.levels below its 64x64 source texels m; n counts the CTA's tiles before it that
+// have a second level. Every thread of the CTA calls it. Levels 3..6 are one warp's work (warp n modulo 8) while the
+// others go on to the next tile. A tile with a second level writes S[n & 1] and meets one barrier; S[n & 1] is written
+// again by the second such tile after it, behind the barrier of the first, which this tile's warp reaches only when it is
+// done. A tile of one level has neither, and the chains of a batch differ, so n must not count it.
 template <typename Tables>
 __device__ __forceinline__ void mip_tile(const MipChain &C, const MipSource &m, int tx, int ty, int n, const Tables &T, MipScratch (&S)[2]) {
     const bool srgb = C.srgb != 0;
@@ -242,14 +243,15 @@ __device__ __forceinline__ void mip_tile(const MipChain &C, const MipSource &m, 
 // the CTA's tiles k = blockIdx.x, + gridDim.x, ...; at(k): the chain and place of tile k
 template <typename Tables, typename At>
 __device__ __forceinline__ void mip_tiles_of_cta(int ntiles, const Tables &T, MipScratch (&S)[2], At &&at) {
-    int n = 0;
-    for (int k = blockIdx.x; k < ntiles; k += gridDim.x, n++) {
+    int n = 0;  // tiles with a second level so far (mip_tile)
+    for (int k = blockIdx.x; k < ntiles; k += gridDim.x) {
         const MipChain *c;
         int x, y;
         at(k, c, x, y);
         const MipSource m = mip_load(*c, x, y);
-        if (n == 0) __syncthreads();  // the tables are staged
+        if (k == (int)blockIdx.x) __syncthreads();  // the tables are staged
         mip_tile(*c, m, x, y, n, T, S);
+        n += c->levels > 1;
     }
 }
 
