@@ -603,6 +603,10 @@ __device__ __forceinline__ void sub_near(const Sub &S, int kind, int b, int l, c
     cost = sub_cost<bc1>(ok ? e : -1, mA, mB, d0, d1, lambda);
 }
 
+// The deciding warp and the three distance-1 warps meet here, after branches that part a warp's lanes: the form that does not
+// ask for converged warps (bar.sync is the aligned one, undefined where a warp's lanes arrive apart).
+__device__ __forceinline__ void near_barrier() { asm volatile("barrier.sync 1, 128;" ::: "memory"); }
+
 struct SubShared {
     uint64_t ring[kWindow];  // the sub-block of the last 16 chosen blocks, slot = block & 15
     __align__(16) int ring_pal[kWindow][8];  // their palettes (palette_word)
@@ -687,7 +691,7 @@ __device__ __forceinline__ void sub_chain(SubShared &M, const Sub S, const SrcU8
                     sub_near<bc1>(S, ck, it, lane, s_tex, s_base, s_bpal, ring, ring_pal, M.dist[0], M.dist[1], lambda, cand, cost, masks);
                     if (lane == 0) { c_cand[it & 1][ck + 1] = cand; M.near_cost[ck] = make_uint2(cost, masks); }
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");  // with the deciding warp
+                near_barrier();  // with the deciding warp
             }
         } else if (warp == R::kDecide) {
             if (it >= 0) {
@@ -707,7 +711,7 @@ __device__ __forceinline__ void sub_chain(SubShared &M, const Sub S, const SrcU8
                     const uint32_t c2 = consider(lane + 35, m2);
                     if (c2 < cost) { cost = c2; masks = m2; order = (uint32_t)lane + 35u; }
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");  // the distance-1 candidates are in
+                near_barrier();  // the distance-1 candidates are in
                 if (lane >= 1 && lane <= 3) {  // orders 1..3
                     const uint2 n = M.near_cost[lane - 1];
                     if (n.x <= cost) { cost = n.x; masks = n.y; order = (uint32_t)lane; }
