@@ -52,10 +52,14 @@ ZTC_API int zap_tex_cuda_version(void);
 ZTC_API const char *zap_tex_cuda_status_string(int status);
 /* the last error message of the calling thread ("" when none) */
 ZTC_API const char *zap_tex_cuda_last_error(void);
-/* creates a context on `device` (its own streams, scratch arena, constant tables); no reference counterpart */
+/* creates a context on `device` (its own streams, scratch pool, constant tables); no reference counterpart. The pool keeps
+   up to 64 MB of the device scratch its calls have used, until reserve names another figure or the context goes;
+   the same holds for a device's default context (ctx == NULL). */
 ZTC_API int zap_tex_cuda_create(int device, zap_tex_cuda_ctx **out);
 ZTC_API int zap_tex_cuda_destroy(zap_tex_cuda_ctx *ctx);
-/* pre-sizes the context's device scratch arena so later _dev calls allocate nothing (e.g. before stream capture) */
+/* sets what the context's scratch pool keeps between calls, and pre-sizes it to that, so later _dev calls that need no more
+   allocate nothing (e.g. before stream capture). A smaller figure than before gives the rest back to the device,
+   0 all of it; the driver holds such memory in steps of 32 MB. */
 ZTC_API int zap_tex_cuda_reserve(zap_tex_cuda_ctx *ctx, size_t scratch_bytes);
 
 /* Kernel tracing, no reference counterpart (the reference times one call with timespec_get, tex_bench.c:208-210).

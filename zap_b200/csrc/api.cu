@@ -106,8 +106,9 @@ struct zap_tex_cuda_ctx {
     cudaMemPool_t pool = nullptr;
     bool owned_default = false;
 };
-// what a pool keeps: the scratch of calls up to 16384x8192 (8 bytes a block); larger scratch is given back
-constexpr uint64_t kPoolKeep = 64ull << 20;
+// what a pool keeps until zap_tex_cuda_reserve names another figure: the scratch of calls up to 16384x8192 (8 bytes a block);
+// larger scratch is given back
+constexpr uint64_t kPoolKeep = 64ull << 20, kPoolStep = 32ull << 20;
 
 namespace {
 
@@ -513,10 +514,14 @@ int zap_tex_cuda_reserve(zap_tex_cuda_ctx *ctx, size_t bytes) {
     ZTC_NVTX();
     int st = resolve(ctx);
     if (st) return st;
-    // _dev calls draw scratch from the context's memory pool: keep that much resident across frees
+    // _dev calls draw scratch from the context's memory pool: keep that much resident across frees, no less and, to a step, no
+    // more (the caller's figure takes the place of kPoolKeep). The driver maps pool memory in steps of 32 MB and gives
+    // back whole steps down to the threshold or below: one of 40 MB kept 32, one of 300 MB 288, one of 8 MB nothing.
     cudaMemPool_t pool = ctx->pool;
     if (!pool) ZTC_CHECK(cudaDeviceGetDefaultMemPool(&pool, ctx->device), "cudaDeviceGetDefaultMemPool");
-    uint64_t keep = ctx->pool && bytes < kPoolKeep ? kPoolKeep : bytes;
+    uint64_t keep = (bytes + kPoolStep - 1) / kPoolStep * kPoolStep, was = 0;
+    ZTC_CHECK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &was), "cudaMemPoolGetAttribute");
+    if (ctx->pool && keep < was) ZTC_CHECK(cudaMemPoolTrimTo(pool, 0), "cudaMemPoolTrimTo");  // what it holds cannot be split
     ZTC_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
     void *p = nullptr;
     ZTC_CHECK(ztc_malloc_async(&p, bytes ? bytes : 1, ctx->stream[0], ctx), "cudaMallocAsync(reserve)");
