@@ -59,7 +59,7 @@ ZTC_API int zap_tex_cuda_create(int device, zap_tex_cuda_ctx **out);
 ZTC_API int zap_tex_cuda_destroy(zap_tex_cuda_ctx *ctx);
 /* sets what the context's scratch pool keeps between calls, and pre-sizes it to that, so later _dev calls that need no more
    allocate nothing (e.g. before stream capture). A smaller figure than before gives the rest back to the device,
-   0 all of it; the driver holds such memory in steps of 32 MB. */
+   0 all of it; the driver holds such memory in steps of 32 MB. A call that fails leaves the figure as it was. */
 ZTC_API int zap_tex_cuda_reserve(zap_tex_cuda_ctx *ctx, size_t scratch_bytes);
 
 /* Kernel tracing, no reference counterpart (the reference times one call with timespec_get, tex_bench.c:208-210).

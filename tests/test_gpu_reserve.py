@@ -47,3 +47,34 @@ def test_reserve_zero_gives_back_what_calls_used(ctx, oracle):
     small = img[:60, :100]
     got = zap_b200.bc_encode_dev(small, zap_b200.BC7, ctx=ctx).cpu().numpy()
     assert np.array_equal(got, oracle.bc_encode(np.ascontiguousarray(small.cpu().numpy()), zap_b200.BC7))
+
+
+@pytest.mark.parametrize("huge", [1 << 62, (1 << 64) - 1])
+def test_reserve_that_fails_changes_nothing(ctx, huge):
+    """A figure beyond the device's memory: what is held stays, and so does the figure that was in force."""
+    img = torch.randint(0, 256, (4096, 8192, 4), dtype=torch.uint8, device="cuda")  # a rate-distortion call uses 128 MB of scratch
+    out = torch.empty(zap_b200.bc_size(8192, 4096, zap_b200.BC7), dtype=torch.uint8, device="cuda")
+    zap_b200.bc_encode_dev(img, zap_b200.BC7, out=out)
+    base = _free()
+    zap_b200.check(zap_b200.load().zap_tex_cuda_reserve(ctx, 64 * MB), "reserve")
+    assert zap_b200.load().zap_tex_cuda_reserve(ctx, huge) != 0
+    assert base - _free() >= 64 * MB
+    zap_b200.bc_encode_rdo_dev(img, zap_b200.BC7, 30.0, band_rows=1, out=out, ctx=ctx)
+    assert base - _free() <= (64 + 4) * MB
+
+
+def test_reserve_without_memory_keeps_the_figure(ctx):
+    """An allocation that fails on the way, made on the host: the figure in force before stays."""
+    lib = zap_b200.load()
+    zap_b200.check(lib.zap_tex_cuda_reserve(ctx, 0), "reserve")
+    base = _free()
+    lib.zap_tex_cuda_debug_fail_allocations(0, 1)
+    try:
+        assert lib.zap_tex_cuda_reserve(ctx, 256 * MB) == -4
+    finally:
+        lib.zap_tex_cuda_debug_fail_allocations(0, 0)
+    img = torch.randint(0, 256, (4096, 8192, 4), dtype=torch.uint8, device="cuda")
+    out = torch.empty(zap_b200.bc_size(8192, 4096, zap_b200.BC7), dtype=torch.uint8, device="cuda")
+    used = base - _free()
+    zap_b200.bc_encode_dev(img, zap_b200.BC7, out=out, ctx=ctx)  # 16 MB of scratch
+    assert base - _free() - used <= 4 * MB

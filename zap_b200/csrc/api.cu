@@ -519,12 +519,19 @@ int zap_tex_cuda_reserve(zap_tex_cuda_ctx *ctx, size_t bytes) {
     // back whole steps down to the threshold or below: one of 40 MB kept 32, one of 300 MB 288, one of 8 MB nothing.
     cudaMemPool_t pool = ctx->pool;
     if (!pool) ZTC_CHECK(cudaDeviceGetDefaultMemPool(&pool, ctx->device), "cudaDeviceGetDefaultMemPool");
+    size_t free_bytes = 0, total = 0;
+    ZTC_CHECK(cudaMemGetInfo(&free_bytes, &total), "cudaMemGetInfo");
+    if (bytes > total) return fail(ZTC_ERR_NO_MEMORY, "reserve: %zu bytes on a device of %zu", bytes, total);
     uint64_t keep = (bytes + kPoolStep - 1) / kPoolStep * kPoolStep, was = 0;
     ZTC_CHECK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &was), "cudaMemPoolGetAttribute");
     if (ctx->pool && keep < was) ZTC_CHECK(cudaMemPoolTrimTo(pool, 0), "cudaMemPoolTrimTo");  // what it holds cannot be split
     ZTC_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
     void *p = nullptr;
-    ZTC_CHECK(ztc_malloc_async(&p, bytes ? bytes : 1, ctx->stream[0], ctx), "cudaMallocAsync(reserve)");
+    const cudaError_t e = ztc_malloc_async(&p, bytes ? bytes : 1, ctx->stream[0], ctx);
+    if (e != cudaSuccess) {  // the figure in force before stays so
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &was);
+        return cuda_fail(e, "cudaMallocAsync(reserve)");
+    }
     ZTC_CHECK(cudaFreeAsync(p, ctx->stream[0]), "cudaFreeAsync(reserve)");
     ZTC_CHECK(cudaStreamSynchronize(ctx->stream[0]), "reserve");
     return ZTC_OK;
