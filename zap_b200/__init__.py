@@ -148,7 +148,6 @@ def bc_encode_dev(t, fmt, out=None, stream=None, ctx=None):
 def bc_encode_rdo_dev(t, fmt, rdo, band_rows=0, out=None, stream=None, ctx=None):
     """Rate-distortion encode (zap_bc_encode with rdo > 0) of an HxWx4 uint8 CUDA tensor: one reference call over
     the whole image (band_rows 0), or one per band of band_rows block rows."""
-    import torch
     w, h, stride = _dev_img(t, (4,))
     if out is None:
         out = _empty_blocks(t, w, h, fmt)
@@ -245,7 +244,6 @@ def bc_merge_dev(planes, fmt, out=None, stream=None, ctx=None):
 
 def bc_encode_split_dev(t, fmt, out=None, stream=None, ctx=None):
     """Encode an HxWx4 uint8 CUDA tensor straight into the split form (the bytes of bc_split(bc_encode(t)))."""
-    import torch
     w, h, stride = _dev_img(t, (4,))
     if out is None:
         out = _empty_blocks(t, w, h, fmt)

@@ -338,7 +338,7 @@ struct Mode6Group {           // a block's shared words
 };
 // returns the SSE; blk: the block (the same in all eight threads)
 __device__ __forceinline__ int mode6_encode_group(Mode6Group &G, uint4 &blk) {
-    const int j = threadIdx.x & 7, c = j & 3, end = j >> 2, base = threadIdx.x & 31 & ~7;
+    const int j = threadIdx.x & 7, c = j & 3, end = j >> 2;
     float mu[4], ax[4];
     pca_axis<4, 1>(TexRef{G.px, 1}, mu, ax);
     float n2 = 0.0f, tl = 1e9f, th = -1e9f;
@@ -436,7 +436,6 @@ __device__ __forceinline__ int mode6_encode_group(Mode6Group &G, uint4 &blk) {
     #pragma unroll
     for (int k = 0; k < 4; k++) { q[0][k] = (int)chan(lo8, k) >> 1; q[1][k] = (int)chan(hi8, k) >> 1; }
     blk = pack_mode6_block(q, pb, (uint64_t)ilo | ((uint64_t)ihi << 32));
-    (void)base;
     return err;
 }
 
@@ -473,8 +472,11 @@ __global__ void __launch_bounds__(8 * kGroupBlocks6) bc7_mode6_group_kernel(SrcU
 // Blocks per SM up to which mode 6 takes eight threads per block. Whole encodes, one / eight threads per block: 64x64 31.2 / 25.4
 // us, 256x256 33.7 / 27.9, 512x512 36.5 / 35.5, 724x724 36.3 / 42.3, 1024x1024 42.3 / 58.7.
 constexpr int kGroupLimit6 = 120;
-// Blocks per SM above which the large CTAs are taken: one wave of small ones is 768. Between that and a wave of
-// large ones (896) the small ones would run a second, nearly empty wave (1918x1077 74.3 -> 68.9 us, 1440x1440 57.9 -> 53.0).
+// Blocks per SM above which the large CTAs are taken: six small CTAs on every SM. An SM holds 896 threads of either size (7
+// or 4 CTAs), but up to six small ones it runs fewer warps side by side and each ends sooner. Whole encodes, large / small
+// CTAs, at so many blocks per SM (592 texels wide, alpha): 520 47.2 / 43.9 us, 704 52.3 / 48.3, 768 52.3 / 49.5, 800 52.3 /
+// 52.3, 864 52.3 / 52.3; 876: 1918x1077 opaque 58.7 / 60.3, 1440x1440 alpha 51.7 / 52.9. Past one wave the small ones lead
+// again for a while (928 60.8 / 58.5, 1152 66.7 / 62.9, 1280 68.7 / 66.9) and then do not (1536 75.3 / 76.2).
 constexpr int kLargeFrom6 = 768;
 // the mode-6 launch, at the CTA size that suits its block count
 cudaError_t launch_mode6(const SrcU8 &src, int bw, int by0, int nblocks, const BlockOut &out, size_t b0, uint32_t *count, uint2 *items,
@@ -863,13 +865,6 @@ __device__ __forceinline__ bool mode1_fits(TexRef ts, const int cand[kMode1Tries
     return false;
 }
 
-ZTC_DEV bool block_opaque(const uint32_t t[16]) {
-    bool opaque = true;
-    #pragma unroll
-    for (int i = 0; i < 16; i++) opaque &= (t[i] >> 24) == 255u;
-    return opaque;
-}
-
 // the group's shared-memory copy of its block (lane l writes texels l and l + 8), for the rolled loops
 __device__ __forceinline__ TexRef stage_group_texels(uint32_t *gtex, const uint32_t t[16], int l, unsigned gmask) {
     __syncwarp(gmask);  // the group's reads of its previous block are done
@@ -979,7 +974,7 @@ template <int KIND>
 __device__ __forceinline__ int m5_part_group(HardBlock &H, int rot, uint32_t q[2], uint32_t &idx) {
     constexpr bool kAlpha = KIND == kPartAlpha;
     constexpr int kBits = kAlpha ? 8 : 7;
-    const int j = threadIdx.x & 7, c = kAlpha ? 0 : min(j & 3, 2), end = j >> 2, base = threadIdx.x & 31 & ~7;
+    const int j = threadIdx.x & 7, c = kAlpha ? 0 : min(j & 3, 2), end = j >> 2;
     const bool own = kAlpha ? (j & 3) == 0 : (j & 3) < 3;  // the thread whose value counts for (channel, endpoint)
     const int i0 = 4 * (j & 3) + 2 * end;
     uint32_t p[2];
@@ -1075,7 +1070,6 @@ __device__ __forceinline__ int m5_part_group(HardBlock &H, int rot, uint32_t q[2
         go = go && (it == 0 || e < err);
         if (go) { err = e; idx = ni; q[0] = n0; q[1] = n1; }
     }
-    (void)base;
     return err;
 }
 // one subset of a mode-1 candidate (pca_endpoints, subset_passes<3, 3>): q: 6 bits a channel, bit 18 of q[0] the p-bit
@@ -1308,8 +1302,7 @@ __global__ void __launch_bounds__(64, ZTC_MINB_BC7_MODE5) bc7_hard_kernel(SrcU8 
     // entries are read 64 at a time (its next 8 rounds) and the opaque ones compacted, so every group has a block
     // while any is left. Each warp runs one mode for long stretches instead of alternating with mode 5 every round
     // (an atlas of 64x64 textures, a quarter of its blocks listed: 0.98 -> 0.80 ms per 2048x2048 encode). After a
-    // single round the blocks are still in shared memory, and group g takes slot g; with one block per CTA, the
-    // whole CTA ranks its partitions and group 0 fits the four best.
+    // single round the blocks are still in shared memory, and group g takes slot g.
     const int g = tid / kBc7Group, l = tid & (kBc7Group - 1);
     const unsigned gmask = 0xFFu << (lane & ~(kBc7Group - 1));
     for (int chunk = 0; (blockIdx.x + 8 * chunk * gridDim.x) * per < n; chunk++) {  // CTA-uniform

@@ -2,7 +2,7 @@
 //
 // RGBA8: with srgb, RGB goes through the sRGB->linear table, the four values are summed left to right and scaled
 // by 0.25f, and the result maps back to sRGB as the first k whose threshold exceeds it (the reference's binary
-// search; here a scan from a per-bucket start, below). Alpha (and RGB without srgb) is (a + b + c + d + 2) >> 2.
+// search; here one table word and no search, srgb_back below). Alpha (and RGB without srgb) is (a + b + c + d + 2) >> 2.
 // Odd sizes drop the last row / column.
 // A launch makes up to six levels of a chain: a CTA takes a 64x64 tile of the source level, from which every texel of
 // levels 1..6 below the tile follows (odd sizes drop the last row or column at each level, and a side of 1 stays
@@ -21,8 +21,6 @@
 
 namespace ztc {
 
-__device__ SrgbTables gSrgb;  // staged into shared memory by each CTA (coalesced loads)
-
 // the bucket of a linear value: 0 below 2^-16 (and for negative values), else its exponent and top 6 mantissa bits
 ZTC_DEV int srgb_bucket(float v) {
     const uint32_t u = f_as_u(v);
@@ -31,7 +29,7 @@ ZTC_DEV int srgb_bucket(float v) {
     return q < kSrgbBuckets - 1 ? q : kSrgbBuckets - 1;
 }
 // first k with v < thr[k] (zap_tex.h:1429-1433), 255 when there is none: the reference's binary search finds it in
-// eight steps; here the scan starts at the bucket's lower bound, one to three steps for the mip generator's values
+// eight steps; here the scan starts at the bucket's lower bound, one to three steps. It builds srgb_back's table.
 ZTC_DEV uint32_t lin_to_srgb(const float *thr, const uint8_t *bucket, float v) {
     int k = bucket[srgb_bucket(v)];
     while (k < 255 && !(v < thr[k])) k++;
@@ -63,6 +61,7 @@ struct MipShared {
     float lin[256];
     uint32_t back[kSrgbBack];
 };
+__device__ MipShared gSrgb;  // what the kernels read of the tables
 struct MipSharedTables {
     uint32_t lin0, back0;  // shared-memory addresses of lin[0] and of back[-kSrgbBackLow]
 #ifdef __CUDACC__
@@ -118,7 +117,7 @@ ZTC_DEV void st_texel(uint8_t *p, uint32_t v) {
 constexpr int kMipTile = 64, kMipThreads = 256, kMipCtas = 4;
 
 // every thread of the CTA calls it; a barrier must follow before the tables are read
-__device__ __forceinline__ void stage_mip_tables(MipShared &S, const SrgbTables *g) {
+__device__ __forceinline__ void stage_mip_tables(MipShared &S, const MipShared *g) {
     for (int k = threadIdx.x; k < 256; k += kMipThreads) S.lin[k] = __ldg(g->lin + k);
     for (int k = threadIdx.x; k < kSrgbBack; k += kMipThreads) S.back[k] = __ldg(g->back + k);
 }
@@ -333,7 +332,10 @@ void srgb_tables_host(SrgbTables &t) {
 cudaError_t upload_mip_tables() {
     SrgbTables T;
     srgb_tables_host(T);
-    return cudaMemcpyToSymbol(gSrgb, &T, sizeof T);
+    MipShared D;
+    std::memcpy(D.lin, T.lin, sizeof D.lin);
+    std::memcpy(D.back, T.back, sizeof D.back);
+    return cudaMemcpyToSymbol(gSrgb, &D, sizeof D);
 }
 
 static int grid_for(long work, int threads) {

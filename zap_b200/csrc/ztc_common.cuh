@@ -17,7 +17,7 @@
 
 // Minimum resident 128-thread CTAs per SM requested from the register allocator, per kernel (tuned on B200:
 // more resident warps hide the latency of these long dependent integer / float chains; see the ncu summaries).
-// Measured again after the kernels changed: BC7 mode 6 at 7 (73 registers; the batch of 64 textures 2119 -> 2106 us against
+// Measured again after the kernels changed: BC7 mode 6 at 7 (72 registers; the batch of 64 textures 2119 -> 2106 us against
 // 6, 5 2142; single images the same at all three), batched mode 1 at 5 (2119 -> 2100 against no limit), mode 5 at 8 (10
 // 2133, 6 2240), BC1 / BC3 at 7 (8 spills: the batch 2147 -> 2118, 1024x1024 BC1 55.1 -> 54.4), BC6H 4 (see bc6_fit);
 // ASTC's single-partition kernel 5 (2048x2048 169.2 us, 4 174, 6 180) in launches of more than one wave, else 4.
