@@ -98,6 +98,7 @@ ZTC_DEV uint32_t box4_srgb(uint32_t a, uint32_t b, uint32_t c, uint32_t d, const
     return ((r[0] >> 16) & 0xFFu) | ((r[1] >> 8) & 0xFF00u) | (r[2] & 0xFF0000u) | (al << 24);
 #endif
 }
+// with the tables in memory: the form the host tests of the arithmetic call
 ZTC_DEV uint32_t box4(uint32_t a, uint32_t b, uint32_t c, uint32_t d, bool srgb, const SrgbTables &T) {
     return srgb ? box4_srgb(a, b, c, d, MipTables{&T}) : box4_linear(a, b, c, d);
 }
